@@ -28,6 +28,7 @@ UNITS = {
     "eik64.cu": ["-fmad=false"],
     "eik32.cu": ["-prec-div=false", "-prec-sqrt=false", "-ftz=true"],
     "surfker.cu": ["-fmad=false"],
+    "surfker_disp.cu": ["-fmad=false"],
     "surfker_group.cu": ["-fmad=false"],
     "util.cu": [],
     "capi.cu": ["-Xcompiler", "-ffp-contract=off"],

@@ -1,11 +1,10 @@
-// Dispersion and depth-kernel kernels: surfdisp96 per surface column,
-// sregn96_hti depth kernels per (column, period), the kernel combination of
-// preproc::combine_kernels, and the host-side layer constants.  Compiled with
+// Depth-kernel kernels: sregn96_hti depth kernels per (column, period), the
+// kernel combination of preproc::combine_kernels, the derivatives of the
+// dispersion roots and the host-side layer constants.  Compiled with
 // -fmad=false (see surfker_dev.cuh).
 // Out of line here, to shrink the instruction footprint: the eigenfunction
 // routines and the complex division (the depth kernel 77 -> 72 -> 68 ms on
-// C3) and dltar4 (the dispersion 141 -> 103 ms).  var, nevill and getsol stay inline (out of line on top of
-// dltar4 they cost more in calls than they save: 107 / 137 / 179 ms).
+// C3) and dltar4.
 #ifndef SK_NOINLINE_EIG
 #define SK_NOINLINE_EIG __noinline__
 #endif
@@ -26,46 +25,6 @@ namespace sa {
 // Kernels
 // ---------------------------------------------------------------------------
 using sk::LayerConst;
-
-// SurfGrid::fwdsurf per column (src/surf_grid.cpp:194-245): one thread per
-// column, periods sequential (surfdisp96's bracket warm start).
-// Resident 64-thread blocks per SM the register allocation is sized for.
-// These kernels are latency-bound FP64 code with per-thread layer arrays in
-// local memory: 10 blocks (96 registers, a few hundred bytes of spills) run
-// the C3 dispersion 1.5x and the depth kernels 1.2x faster than the
-// unconstrained allocation (128 / 202 registers), and put the 90,601 C3
-// columns in one wave.
-// Grids with more columns than one wave at 10 blocks per SM take the
-// 16-block form (64 registers, a few more spills): with several waves the
-// extra warps hide more FP64 latency (C5, 361,201 columns: 700 -> 659 ms),
-// while a one-wave grid gains no warps and only pays the spills (C3: 122 ->
-// 134 ms).  Both forms compute the same bits.
-template <int MINB>
-__global__ void __launch_bounds__(64, MINB)
-surfdisp_columns_kernel(int nx, int ny, int nz, const double* __restrict__ vs3d, int nper,
-                        const double* __restrict__ periods, int iflsph, int iwave, int igr,
-                        const LayerConst* __restrict__ Lp, double* svel, int* status) {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= nx * ny) return;
-    const LayerConst& L = *Lp;
-    const int ix = col / ny, iy = col % ny;
-    float vp[sk::MMAX], vs[sk::MMAX], rho[sk::MMAX];
-    sk::column_model(vs3d + (size_t)col * nz, nz, L, vp, vs, rho);
-    double t[sk::KMAX], cg[sk::KMAX];
-    for (int i = 0; i < nper; i++) {
-        t[i] = periods[i];
-        cg[i] = 0.0;
-    }
-    // SK_DISP_SERIAL builds the searches in the Fortran's call structure
-    // (same bits; 1.2-1.3x slower, lanes diverge across the call sites)
-#ifdef SK_DISP_SERIAL
-    const int st = sk::surfdisp96(L, vp, vs, rho, iflsph, iwave, 1, igr, nper, t, cg);
-#else
-    const int st = sk::surfdisp96_lockstep(L, vp, vs, rho, iflsph, iwave, igr, nper, t, cg);
-#endif
-    if (status) status[ix + nx * iy] = st;
-    for (int ip = 0; ip < nper; ip++) svel[(size_t)ip * nx * ny + ix + (size_t)nx * iy] = cg[ip];
-}
 
 // The correctly rounded transcendentals on device arrays (sa_math_eval):
 // f = 0 exp, 1 log, 2 sin, 3 cos, 4 sincos (y holds sin, cos pairs), 5
@@ -388,7 +347,6 @@ dispersion_dcdvs_kernel(int nx, int ny, int nz, const double* __restrict__ vs3d,
         M.b[i] = (float)(vs[i] * L.sd_tmp[i]);
         M.rho[i] = rho[i] * L.sd_rhofac[i];
     }
-    M.del1st = 0.0;
     double ein[5 * sk::MMAX], logn[sk::MMAX], db[sk::MMAX], da[sk::MMAX], dr[sk::MMAX];
     const double c = svel[(size_t)ip * nx * ny + ix + (size_t)nx * iy];
     sk::root_dcdm(M, periods[ip], c, db, da, dr, ein, logn);
@@ -449,24 +407,6 @@ cudaError_t launch_combine_vs_derivative(int nx, int ny, int nz, int nper, const
     combine_vs_derivative_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(
         nx, ny, nz, nper, adj_s, vs3d, vp3d, sen_vs, sen_vp, sen_rho, sen_hs, area_row,
         reinterpret_cast<const LayerConst*>(layer_const), grad);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_surfdisp_columns(int nx, int ny, int nz, const double* vs3d, int nper,
-                                    const double* periods, int iflsph, int iwave, int igr,
-                                    const void* layer_const, double* svel, int* status,
-                                    cudaStream_t st) {
-    const int n = nx * ny;
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const LayerConst* Lp = reinterpret_cast<const LayerConst*>(layer_const);
-    if (n > nsm * 10 * 64)
-        surfdisp_columns_kernel<16><<<(n + 63) / 64, 64, 0, st>>>(
-            nx, ny, nz, vs3d, nper, periods, iflsph, iwave, igr, Lp, svel, status);
-    else
-        surfdisp_columns_kernel<10><<<(n + 63) / 64, 64, 0, st>>>(
-            nx, ny, nz, vs3d, nper, periods, iflsph, iwave, igr, Lp, svel, status);
     return cudaGetLastError();
 }
 

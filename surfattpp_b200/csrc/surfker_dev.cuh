@@ -1,5 +1,5 @@
 // Device routines of the dispersion and depth-kernel engine, shared by
-// surfker.cu and surfker_group.cu.
+// surfker.cu, surfker_disp.cu and surfker_group.cu.
 //
 // Dispersion and depth-kernel engine: surfdisp96 (Rayleigh/Love phase or
 // group velocity root search) per surface column and sregn96_hti (Rayleigh
@@ -50,18 +50,14 @@ struct LayerConst {
 // (smaller instruction footprint, bit-identical results); surfker_group.cu
 // keeps everything inline, because with layer_integrals out of line the
 // group-velocity kernel's saved first-evaluation kernels come back
-// overwritten on the device (see surfker_group.cu).  SK_NOINLINE marks the
-// routines that stay inline everywhere
-// (dltar1, nevill, getsol: out of line they cost more than they save).
-#ifndef SK_NOINLINE
-#define SK_NOINLINE inline
-#endif
+// overwritten on the device (see surfker_group.cu).
 // The eigenfunction routines (varsv, dnka_rg, evalg, layer_integrals): out of
 // line in surfker.cu (SK_NOINLINE_EIG set there), inline elsewhere.
 #ifndef SK_NOINLINE_EIG
 #define SK_NOINLINE_EIG inline
 #endif
-// dltar4: out of line in surfker.cu (SK_ATTR_DLTAR4 set there).
+// dltar4: out of line in surfker.cu and surfker_disp.cu (SK_ATTR_DLTAR4 set
+// there).
 #ifndef SK_ATTR_DLTAR4
 #define SK_ATTR_DLTAR4 inline
 #endif
@@ -86,6 +82,17 @@ static __device__ SK_MATH_ATTR double sk_log(double x) { return cr::log(x); }
 
 __device__ __forceinline__ double dsign1(double x) { return copysign(1.0, x); }
 
+// a / b rounded to nearest from rh = RN(1/b) and rl = recip_lo(b, rh), about
+// 1/b - rh: RN(a rh + a rl) lies within an ulp of a / b, its remainder is
+// exact, and one correction by rh rounds correctly (Markstein, IBM J. Res.
+// Dev. 34(1) 1990); for |a| above 2^-900 or 0.  Four operations where
+// several quotients share a divisor, against about ten of a division.
+__device__ __forceinline__ double recip_lo(double b, double rh) { return fma(-rh, b, 1.0) * rh; }
+__device__ __forceinline__ double quot(double a, double b, double rh, double rl) {
+    const double q = fma(a, rh, a * rl);
+    return fma(fma(-q, b, a), rh, q);
+}
+
 // Brocher relations, scalar forms (include/utils.h:185-187, :223-225)
 __device__ __forceinline__ double vs2vp(double vs) {
     return 0.9409 + 2.0947 * vs - 0.8206 * vs * vs + 0.2683 * vs * vs * vs - 0.0251 * vs * vs * vs * vs;
@@ -105,16 +112,15 @@ __device__ __forceinline__ double dalpha_dbeta(double vs) {
 
 // Float layer model of one column: build_disp_req (src/surfdisp.cpp:60-108)
 // with the Brocher branch of SurfGrid::fwdsurf (src/surf_grid.cpp:214-226).
+__device__ __forceinline__ void layer_model(double b, float& vp, float& vs, float& rho) {
+    const double a = vs2vp(b);
+    vs = (float)b;
+    vp = (float)a;
+    rho = (float)vp2rho(a);
+}
 __device__ inline void column_model(const double* vs1d, int nz, const LayerConst& L, float* vp,
                                     float* vs, float* rho) {
-    for (int kk = 0; kk < nz; ++kk) {
-        const double b = vs1d[kk];
-        const double a = vs2vp(b);
-        const double r = vp2rho(a);
-        vs[kk] = (float)b;
-        vp[kk] = (float)a;
-        rho[kk] = (float)r;
-    }
+    for (int kk = 0; kk < nz; ++kk) layer_model(vs1d[kk], vp[kk], vs[kk], rho[kk]);
     vs[nz] = vs[nz - 1];
     vp[nz] = vp[nz - 1];
     rho[nz] = rho[nz - 1];
@@ -126,7 +132,6 @@ __device__ inline void column_model(const double* vs1d, int nz, const LayerConst
 struct SDModel {
     int mmax, llw;
     float d[MMAX], a[MMAX], b[MMAX], rho[MMAX];
-    double del1st;
 };
 
 struct VarOut {
@@ -193,9 +198,12 @@ __device__ inline VarOut var(double p, double q, double ra, double rb, double wv
 
 // surfdisp96.f:1054-1098: the 5x5 compound layer matrix, ca[j][i] holding
 // the Fortran ca(j+1, i+1).
-__device__ inline void dnka_matrix(double ca[5][5], double wvno2, double gam, double gammk,
-                                   double rho, const VarOut& v) {
+// rr = RN(1/rho); r2 = RN(1/rho^2), or 0 to divide by rho^2 instead.
+__device__ __forceinline__ void dnka_matrix(double ca[5][5], double wvno2, double gam,
+                                            double gammk, double rho, const VarOut& v, double rr,
+                                            double r2 = 0.0) {
     const double one = 1.0, two = 2.0;
+    const double rl = recip_lo(rho, rr);
     const double gamm1 = gam - one;
     const double twgm1 = gam + gamm1;
     const double gmgmk = gam * gammk;
@@ -204,10 +212,11 @@ __device__ inline void dnka_matrix(double ca[5][5], double wvno2, double gam, do
     const double rho2 = rho * rho;
     const double a0pq = v.a0 - v.cpcq;
     ca[0][0] = v.cpcq - two * gmgm1 * a0pq - gmgmk * v.xz - wvno2 * gm1sq * v.wy;
-    ca[0][1] = (wvno2 * v.cpy - v.cqx) / rho;
-    ca[0][2] = -((twgm1 * a0pq + gammk * v.xz + wvno2 * gamm1 * v.wy) / rho);
-    ca[0][3] = (v.cpz - wvno2 * v.cqw) / rho;
-    ca[0][4] = -((two * wvno2 * a0pq + v.xz + wvno2 * wvno2 * v.wy) / rho2);
+    ca[0][1] = quot(wvno2 * v.cpy - v.cqx, rho, rr, rl);
+    ca[0][2] = -quot(twgm1 * a0pq + gammk * v.xz + wvno2 * gamm1 * v.wy, rho, rr, rl);
+    ca[0][3] = quot(v.cpz - wvno2 * v.cqw, rho, rr, rl);
+    const double s04 = two * wvno2 * a0pq + v.xz + wvno2 * wvno2 * v.wy;
+    ca[0][4] = -(r2 != 0.0 ? quot(s04, rho2, r2, recip_lo(rho2, r2)) : s04 / rho2);
     ca[1][0] = (gmgmk * v.cpz - gm1sq * v.cqw) * rho;
     ca[1][1] = v.cpcq;
     ca[1][2] = gammk * v.cpz - gamm1 * v.cqw;
@@ -236,7 +245,7 @@ __device__ inline void dnka_matrix(double ca[5][5], double wvno2, double gam, do
 __device__ inline void dnka_apply(const double* e, double* ee, double wvno2, double gam,
                                   double gammk, double rho, const VarOut& v) {
     double ca[5][5];
-    dnka_matrix(ca, wvno2, gam, gammk, rho, v);
+    dnka_matrix(ca, wvno2, gam, gammk, rho, v, 1.0 / rho);
 #pragma unroll
     for (int i = 0; i < 5; i++) {
         double cr = 0.0;
@@ -252,11 +261,8 @@ __device__ __forceinline__ void normc(double* ee, int n) {
     for (int i = 0; i < n; i++)
         if (fabs(ee[i]) > t1) t1 = fabs(ee[i]);
     if (t1 < 1.e-40) t1 = 1.0;
-    for (int i = 0; i < n; i++) {
-        double t2 = ee[i];
-        t2 = t2 / t1;
-        ee[i] = t2;
-    }
+    const double rh = 1.0 / t1, rl = recip_lo(t1, rh);
+    for (int i = 0; i < n; i++) ee[i] = quot(ee[i], t1, rh, rl);
 }
 
 // surfdisp96.f:801-901
@@ -322,7 +328,7 @@ static __device__ SK_ATTR_DLTAR4 double dltar4(const SDModel& M, double wvno, do
 }
 
 // surfdisp96.f:737-797
-__device__ SK_NOINLINE double dltar1(const SDModel& M, double wvno, double omega) {
+__device__ inline double dltar1(const SDModel& M, double wvno, double omega) {
     const int mmax = M.mmax;
     double beta1 = (double)M.b[mmax - 1];
     double rho1 = (double)M.rho[mmax - 1];
@@ -393,7 +399,7 @@ __device__ inline void layer_matrix(double a, double b, double rho, double d, do
     const double ra = sqrt((wvno + xka) * fabs(wvno - xka));
     const double rb = sqrt((wvno + xkb) * fabs(wvno - xkb));
     const VarOut v = var(ra * d, rb * d, ra, rb, wvno, xka, xkb, d);
-    dnka_matrix(ca, wvno2, gam, gammk, rho, v);
+    dnka_matrix(ca, wvno2, gam, gammk, rho, v, 1.0 / rho);
 }
 __device__ inline void halfspace_vector(double a, double b, double rho, double wvno, double omega,
                                         double e[5]) {
@@ -491,121 +497,6 @@ __device__ __forceinline__ double dltar(const SDModel& M, double wvno, double om
     return kk == 1 ? dltar1(M, wvno, omega) : dltar4(M, wvno, omega);
 }
 
-// surfdisp96.f:578-711 (nevill with half inlined)
-__device__ SK_NOINLINE double nevill(const SDModel& M, double t, double c1, double c2, double del1,
-                                double del2, int ifunc, double twopi) {
-    double x[20], y[20];
-    const double omega = twopi / t;
-    double c3 = 0.5 * (c1 + c2);
-    double del3 = dltar(M, omega / c3, omega, ifunc);
-    int nev = 1;
-    int nctrl = 1;
-    int m = 1;
-    const double p01 = (double)0.01f;
-    for (;;) {
-        nctrl = nctrl + 1;
-        if (nctrl >= 100) break;
-        if (c3 < fmin(c1, c2) || c3 > fmax(c1, c2)) {
-            nev = 0;
-            c3 = 0.5 * (c1 + c2);
-            del3 = dltar(M, omega / c3, omega, ifunc);
-        }
-        const double s13 = del1 - del3;
-        const double s32 = del3 - del2;
-        if (dsign1(del3) * dsign1(del1) < 0.0) {
-            c2 = c3;
-            del2 = del3;
-        } else {
-            c1 = c3;
-            del1 = del3;
-        }
-        if (fabs(c1 - c2) <= 1.e-6 * c1) break;
-        if (dsign1(s13) != dsign1(s32)) nev = 0;
-        const double ss1 = fabs(del1);
-        const double s1 = p01 * ss1;
-        const double ss2 = fabs(del2);
-        const double s2 = p01 * ss2;
-        if (s1 > ss2 || s2 > ss1 || nev == 0) {
-            c3 = 0.5 * (c1 + c2);
-            del3 = dltar(M, omega / c3, omega, ifunc);
-            nev = 1;
-            m = 1;
-        } else {
-            if (nev == 2) {
-                x[m] = c3;
-                y[m] = del3;
-            } else {
-                x[0] = c1;
-                y[0] = del1;
-                x[1] = c2;
-                y[1] = del2;
-                m = 1;
-            }
-            bool bad = false;
-            for (int kk = 1; kk <= m; kk++) {
-                const int j = m - kk + 1;
-                const double denom = y[m] - y[j - 1];
-                if (fabs(denom) < 1.0e-10 * fabs(y[m])) {
-                    bad = true;
-                    break;
-                }
-                x[j - 1] = (-(y[j - 1] * x[j]) + y[m] * x[j - 1]) / denom;
-            }
-            if (!bad) {
-                c3 = x[0];
-                del3 = dltar(M, omega / c3, omega, ifunc);
-                nev = 2;
-                m = m + 1;
-                if (m > 10) m = 10;
-            } else {
-                c3 = 0.5 * (c1 + c2);
-                del3 = dltar(M, omega / c3, omega, ifunc);
-                nev = 1;
-                m = 1;
-            }
-        }
-    }
-    return c3;
-}
-
-// surfdisp96.f:403-498
-__device__ SK_NOINLINE int getsol(SDModel& M, double t1, double& c1, double clow, double dc, double cm,
-                             float betmx, int ifunc, int ifirst) {
-    const double twopi = 2.0 * 3.141592653589793;
-    double omega = twopi / t1;
-    double wvno = omega / c1;
-    double del1 = dltar(M, wvno, omega, ifunc);
-    if (ifirst == 1) M.del1st = del1;
-    const double plmn = dsign1(M.del1st) * dsign1(del1);
-    int idir;
-    if (ifirst == 1) idir = +1;
-    else if (plmn >= 0.0) idir = +1;
-    else idir = -1;
-    for (int guard = 0; guard < 100000; guard++) {
-        double c2;
-        if (idir > 0) c2 = c1 + dc;
-        else c2 = c1 - dc;
-        if (c2 <= clow) {
-            idir = +1;
-            c1 = clow;
-            continue;
-        }
-        omega = twopi / t1;
-        wvno = omega / c2;
-        const double del2 = dltar(M, wvno, omega, ifunc);
-        if (dsign1(del1) != dsign1(del2)) {
-            c1 = nevill(M, t1, c1, c2, del1, del2, ifunc, twopi);
-            if (c1 > (double)betmx) return -1;
-            return 1;
-        }
-        c1 = c2;
-        del1 = del2;
-        if (c1 < cm) return -1;
-        if (c1 >= ((double)betmx + dc)) return -1;
-    }
-    return -1;
-}
-
 // surfdisp96.f:380-401 (REAL*4)
 __device__ inline float gtsolh(float a, float b) {
     float c = 0.95f * b;
@@ -626,439 +517,66 @@ __device__ inline float gtsolh(float a, float b) {
     return c;
 }
 
-// surfdisp96.f:57-373 up to the root searches: the (flattened) layer model,
-// the bracket step dc and the starting velocity cc of the first search.
-__device__ inline void sd_setup(const LayerConst& L, const float* vpm, const float* vsm,
-                                const float* rhom, int iflsph, int iwave, SDModel& M,
-                                float& betmx, double& cc, double& dc) {
-    const int mmax = L.mmax;
-    M.mmax = mmax;
-    float vmin = vsm[0];
-    for (int i = 1; i < mmax; i++) vmin = fminf(vmin, vsm[i]);
-    float ddc0;
-    if (vmin < 1.0f) ddc0 = 0.001f;
-    else if (vmin < 2.0f) ddc0 = 0.002f;
-    else ddc0 = 0.005f;
-    M.llw = 1;
-    if (vsm[0] <= 0.0f) M.llw = 2;
-    for (int i = 0; i < mmax; i++) {
-        if (iflsph == 1) {   // sphere(0,0): velocities and thickness flattened
-            M.d[i] = L.sd_d[i];
-            M.a[i] = (float)(vpm[i] * L.sd_tmp[i]);
-            M.b[i] = (float)(vsm[i] * L.sd_tmp[i]);
-        } else {
-            M.d[i] = L.thk[i];
-            M.a[i] = vpm[i];
-            M.b[i] = vsm[i];
-        }
-        M.rho[i] = rhom[i];
+// surfdisp96.f:57-373 up to the root searches: sphere(0, 0) and the density
+// mapping sphere(ifunc, 1) of one layer;
+__device__ __forceinline__ void flatten_layer(const LayerConst& L, int i, int iflsph, bool love,
+                                              float vp, float vs, float rho, float& fd, float& fa,
+                                              float& fb, float& fr) {
+    if (iflsph == 1) {
+        fd = L.sd_d[i];
+        fa = (float)(vp * L.sd_tmp[i]);
+        fb = (float)(vs * L.sd_tmp[i]);
+        fr = rho * (love ? L.sd_rhofac_love[i] : L.sd_rhofac[i]);
+    } else {
+        fd = L.thk[i];
+        fa = vp;
+        fb = vs;
+        fr = rho;
     }
-    M.del1st = 0.0;
+}
+// and from the flattened layers and the smallest unflattened velocity the
+// bracket step dc and the starting velocity cc of the first search.
+__device__ inline void first_velocity(int mmax, float vmin, const float* a, const float* b,
+                                      float& betmx, double& cc, double& dc) {
+    float ddc;
+    if (vmin < 1.0f) ddc = 0.001f;
+    else if (vmin < 2.0f) ddc = 0.002f;
+    else ddc = 0.005f;
     int jmn = 1, jsol = 1;
     float betmn = 1.e20f;
     betmx = -1.e20f;
     for (int i = 0; i < mmax; i++) {
-        if (M.b[i] > 0.01f && M.b[i] < betmn) {
-            betmn = M.b[i];
+        if (b[i] > 0.01f && b[i] < betmn) {
+            betmn = b[i];
             jmn = i + 1;
             jsol = 1;
-        } else if (M.b[i] <= 0.01f && M.a[i] < betmn) {
-            betmn = M.a[i];
+        } else if (b[i] <= 0.01f && a[i] < betmn) {
+            betmn = a[i];
             jmn = i + 1;
             jsol = 0;
         }
-        if (M.b[i] > betmx) betmx = M.b[i];
+        if (b[i] > betmx) betmx = b[i];
     }
-    const int ifunc = (iwave == 1) ? 1 : 2;
-    if (iflsph == 1)   // sphere(ifunc,1): density mapping
-        for (int i = 0; i < mmax; i++)
-            M.rho[i] = rhom[i] * (ifunc == 1 ? L.sd_rhofac_love[i] : L.sd_rhofac[i]);
-    const float ddc = ddc0;
     float cc1;
     if (jsol == 0) cc1 = betmn;
-    else cc1 = gtsolh(M.a[jmn - 1], M.b[jmn - 1]);
+    else cc1 = gtsolh(a[jmn - 1], b[jmn - 1]);
     cc1 = 0.95f * cc1;
     cc1 = 0.90f * cc1;
     cc = (double)cc1;
     dc = fabs((double)ddc);
 }
-
-// surfdisp96.f:57-373 for one column, the searches in the reference's
-// order.  vp/vs/rho: unflattened float model (mmax layers).  Returns 0, or
-// 1 when the fundamental-mode search fails.
-static __device__ int surfdisp96(const LayerConst& L, const float* vpm, const float* vsm,
-                          const float* rhom, int iflsph, int iwave, int mode, int igr, int kmax,
-                          const double* t, double* cg) {
-    SDModel M;
-    float betmx;
-    double cc, dc;
-    sd_setup(L, vpm, vsm, rhom, iflsph, iwave, M, betmx, cc, dc);
-    const int ifunc = (iwave == 1) ? 1 : 2;
-    const double one = 1.0e-2;
-    const float sone = 1.500f;
-    const float h = 0.005f;
-    const double onea = (double)sone;
-    double c[KMAX], cb[KMAX];
-    double c1 = cc;
-    const double cm = cc;
-    double clow = cc;
-    for (int i = 0; i < kmax; i++) {
-        cb[i] = 0.0;
-        c[i] = 0.0;
+__device__ inline void sd_setup(const LayerConst& L, const double* vs1d, int nz, int iflsph,
+                                int iwave, SDModel& M, float& betmx, double& cc, double& dc) {
+    M.mmax = L.mmax;
+    float vmin = 0.0f;
+    for (int i = 0; i < L.mmax; i++) {
+        float vp, vs, rho;
+        layer_model(vs1d[min(i, nz - 1)], vp, vs, rho);
+        if (i == 0) M.llw = vs <= 0.0f ? 2 : 1;
+        vmin = i == 0 ? vs : fminf(vmin, vs);
+        flatten_layer(L, i, iflsph, iwave == 1, vp, vs, rho, M.d[i], M.a[i], M.b[i], M.rho[i]);
     }
-    int ift = 999;
-    for (int iq = 1; iq <= mode; iq++) {
-        int kfail = -1;
-        for (int k = 1; k <= kmax; k++) {
-            if (k >= ift) {
-                kfail = k;
-                break;
-            }
-            double t1 = t[k - 1];
-            float t1a, t1b = 0.0f;
-            if (igr > 0) {
-                t1a = (float)(t1 / (double)(1.0f + h));
-                t1b = (float)(t1 / (double)(1.0f - h));
-                t1 = (double)t1a;
-            } else {
-                t1a = (float)t1;
-            }
-            int ifirst;
-            if (k == 1 && iq == 1) {
-                c1 = cc;
-                clow = cc;
-                ifirst = 1;
-            } else if (k == 1 && iq > 1) {
-                c1 = c[0] + one * dc;
-                clow = c1;
-                ifirst = 1;
-            } else if (k > 1 && iq > 1) {
-                ifirst = 0;
-                clow = c[k - 1] + one * dc;
-                c1 = c[k - 2];
-                if (c1 < clow) c1 = clow;
-            } else {
-                ifirst = 0;
-                c1 = c[k - 2] - onea * dc;
-                clow = cm;
-            }
-            int iret = getsol(M, t1, c1, clow, dc, cm, betmx, ifunc, ifirst);
-            if (iret == -1) {
-                kfail = k;
-                break;
-            }
-            c[k - 1] = c1;
-            if (igr > 0) {
-                t1 = (double)t1b;
-                ifirst = 0;
-                clow = cb[k - 1] + one * dc;
-                c1 = c1 - onea * dc;
-                iret = getsol(M, t1, c1, clow, dc, cm, betmx, ifunc, ifirst);
-                if (iret == -1) c1 = c[k - 1];
-                cb[k - 1] = c1;
-            } else {
-                c1 = 0.0;
-            }
-            const float cc0 = (float)c[k - 1];
-            const float ccg = (float)c1;
-            if (igr == 0) {
-                cg[k - 1] = cc0;
-            } else {
-                const float gvel =
-                    (1.0f / t1a - 1.0f / t1b) / (1.0f / (t1a * cc0) - 1.0f / (t1b * ccg));
-                cg[k - 1] = gvel;
-            }
-        }
-        if (kfail < 0) continue;
-        for (int i = kfail; i <= kmax; i++) cg[i - 1] = 0.0;
-        if (iq <= 1) return 1;
-        ift = kfail;
-    }
-    return 0;
-}
-
-// surfdisp96's fundamental-mode searches (getsol's bracket march, nevill's
-// refinement, the period loop and the group velocity's second search) as a
-// resumable state machine: advance() runs the control flow up to the next
-// secular-function evaluation, leaves the requested (wvno, omega) in the
-// state and returns true; the caller evaluates dltar there and passes the
-// value back at the next advance().  Each lane's sequence of evaluations,
-// and every operation on their values, are those of surfdisp96() above (the
-// same trial velocities, brackets and Neville tables), so the results are
-// bit-identical; what changes is that all lanes of a warp meet at one dltar
-// call site, whichever period, march step or refinement step each is in,
-// instead of running the march and the refinements of differently long
-// brackets one after another.  Only mode 1 (the fundamental mode, what every
-// caller here asks for).
-struct RootSearch {
-    enum : int { kStart = 0, kGsFirst, kGsMarch, kGsStep, kNvFirst, kNvTop, kNvTopEval,
-                 kNvMid, kNvEnd, kDone };
-    // per column
-    double cc, dc, cm;
-    float betmx;
-    int igr, kmax;
-    // progress
-    int ph, k, stage, status;
-    float t1a, t1b;
-    double cprev;                      // c(k-1) of the period before
-    double ck;                         // this period's phase velocity
-    // getsol
-    double t1, c1, clow, del1, c2;
-    int idir, guard, ifirst;
-    // nevill
-    double n1, n2, nd1, nd2, c3, del3, nomega;
-    int nev, nctrl, m;
-    double x[11], y[11];
-    // the requested evaluation
-    double wvno, omega;
-};
-
-// surfdisp96.f:57-373 period loop, one step (see RootSearch).
-__device__ inline bool root_advance(RootSearch& S, SDModel& M, double del, const double* t,
-                                    double* cg) {
-    const double twopi = 2.0 * 3.141592653589793;
-    const double one = 1.0e-2;
-    const double onea = (double)1.500f;
-    const float h = 0.005f;
-    for (;;) {
-        switch (S.ph) {
-            case RootSearch::kStart: {   // next period (surfdisp96.f:121-160)
-                S.k++;
-                if (S.k > S.kmax) {
-                    S.ph = RootSearch::kDone;
-                    S.status = 0;
-                    return false;
-                }
-                double t1 = t[S.k - 1];
-                S.t1b = 0.0f;
-                if (S.igr > 0) {
-                    S.t1a = (float)(t1 / (double)(1.0f + h));
-                    S.t1b = (float)(t1 / (double)(1.0f - h));
-                    t1 = (double)S.t1a;
-                } else {
-                    S.t1a = (float)t1;
-                }
-                if (S.k == 1) {
-                    S.c1 = S.cc;
-                    S.clow = S.cc;
-                    S.ifirst = 1;
-                } else {
-                    S.ifirst = 0;
-                    S.c1 = S.cprev - onea * S.dc;
-                    S.clow = S.cm;
-                }
-                S.t1 = t1;
-                S.stage = 0;
-                // getsol entry: del1 at c1 (surfdisp96.f:413-416)
-                S.omega = twopi / S.t1;
-                S.wvno = S.omega / S.c1;
-                S.ph = RootSearch::kGsFirst;
-                return true;
-            }
-            case RootSearch::kGsFirst: {
-                S.del1 = del;
-                if (S.ifirst == 1) M.del1st = S.del1;
-                const double plmn = dsign1(M.del1st) * dsign1(S.del1);
-                if (S.ifirst == 1) S.idir = +1;
-                else if (plmn >= 0.0) S.idir = +1;
-                else S.idir = -1;
-                S.guard = 0;
-                S.ph = RootSearch::kGsMarch;
-                break;
-            }
-            case RootSearch::kGsMarch: {   // next trial velocity (surfdisp96.f:431-446)
-                if (S.guard >= 100000) goto getsol_fail;
-                if (S.idir > 0) S.c2 = S.c1 + S.dc;
-                else S.c2 = S.c1 - S.dc;
-                if (S.c2 <= S.clow) {
-                    S.idir = +1;
-                    S.c1 = S.clow;
-                    S.guard++;
-                    break;
-                }
-                S.omega = twopi / S.t1;
-                S.wvno = S.omega / S.c2;
-                S.ph = RootSearch::kGsStep;
-                return true;
-            }
-            case RootSearch::kGsStep: {
-                const double del2 = del;
-                if (dsign1(S.del1) != dsign1(del2)) {
-                    // nevill entry (surfdisp96.f:578-590)
-                    S.n1 = S.c1;
-                    S.n2 = S.c2;
-                    S.nd1 = S.del1;
-                    S.nd2 = del2;
-                    S.nomega = twopi / S.t1;
-                    S.c3 = 0.5 * (S.n1 + S.n2);
-                    S.omega = S.nomega;
-                    S.wvno = S.nomega / S.c3;
-                    S.ph = RootSearch::kNvFirst;
-                    return true;
-                }
-                S.c1 = S.c2;
-                S.del1 = del2;
-                if (S.c1 < S.cm) goto getsol_fail;
-                if (S.c1 >= ((double)S.betmx + S.dc)) goto getsol_fail;
-                S.guard++;
-                S.ph = RootSearch::kGsMarch;
-                break;
-            }
-            case RootSearch::kNvFirst:
-                S.del3 = del;
-                S.nev = 1;
-                S.nctrl = 1;
-                S.m = 1;
-                S.ph = RootSearch::kNvTop;
-                break;
-            case RootSearch::kNvTop:   // surfdisp96.f:593-600
-                S.nctrl = S.nctrl + 1;
-                if (S.nctrl >= 100) goto nevill_done;
-                if (S.c3 < fmin(S.n1, S.n2) || S.c3 > fmax(S.n1, S.n2)) {
-                    S.nev = 0;
-                    S.c3 = 0.5 * (S.n1 + S.n2);
-                    S.omega = S.nomega;
-                    S.wvno = S.nomega / S.c3;
-                    S.ph = RootSearch::kNvTopEval;
-                    return true;
-                }
-                S.ph = RootSearch::kNvMid;
-                break;
-            case RootSearch::kNvTopEval:
-                S.del3 = del;
-                S.ph = RootSearch::kNvMid;
-                break;
-            case RootSearch::kNvMid: {   // surfdisp96.f:601-696
-                const double s13 = S.nd1 - S.del3;
-                const double s32 = S.del3 - S.nd2;
-                if (dsign1(S.del3) * dsign1(S.nd1) < 0.0) {
-                    S.n2 = S.c3;
-                    S.nd2 = S.del3;
-                } else {
-                    S.n1 = S.c3;
-                    S.nd1 = S.del3;
-                }
-                if (fabs(S.n1 - S.n2) <= 1.e-6 * S.n1) goto nevill_done;
-                if (dsign1(s13) != dsign1(s32)) S.nev = 0;
-                const double p01 = (double)0.01f;
-                const double ss1 = fabs(S.nd1);
-                const double s1 = p01 * ss1;
-                const double ss2 = fabs(S.nd2);
-                const double s2 = p01 * ss2;
-                bool halve = s1 > ss2 || s2 > ss1 || S.nev == 0;
-                if (!halve) {
-                    int m = S.m;
-                    if (S.nev == 2) {
-                        S.x[m] = S.c3;
-                        S.y[m] = S.del3;
-                    } else {
-                        S.x[0] = S.n1;
-                        S.y[0] = S.nd1;
-                        S.x[1] = S.n2;
-                        S.y[1] = S.nd2;
-                        m = 1;
-                    }
-                    bool bad = false;
-                    for (int kk = 1; kk <= m; kk++) {
-                        const int j = m - kk + 1;
-                        const double denom = S.y[m] - S.y[j - 1];
-                        if (fabs(denom) < 1.0e-10 * fabs(S.y[m])) {
-                            bad = true;
-                            break;
-                        }
-                        S.x[j - 1] = (-(S.y[j - 1] * S.x[j]) + S.y[m] * S.x[j - 1]) / denom;
-                    }
-                    if (!bad) {
-                        S.c3 = S.x[0];
-                        S.nev = 2;
-                        m = m + 1;
-                        if (m > 10) m = 10;
-                        S.m = m;
-                    } else {
-                        halve = true;
-                    }
-                }
-                if (halve) {
-                    S.c3 = 0.5 * (S.n1 + S.n2);
-                    S.nev = 1;
-                    S.m = 1;
-                }
-                S.omega = S.nomega;
-                S.wvno = S.nomega / S.c3;
-                S.ph = RootSearch::kNvEnd;
-                return true;
-            }
-            case RootSearch::kNvEnd:
-                S.del3 = del;
-                S.ph = RootSearch::kNvTop;
-                break;
-            default:
-                return false;
-        }
-        continue;
-    nevill_done:   // getsol after nevill (surfdisp96.f:455-459)
-        S.c1 = S.c3;
-        if (S.c1 > (double)S.betmx) goto getsol_fail;
-        // getsol found its root: c1
-        if (S.stage == 0) {
-            S.ck = S.c1;
-            if (S.igr > 0) {   // the group velocity's second search (surfdisp96.f:181-192)
-                S.stage = 1;
-                S.t1 = (double)S.t1b;
-                S.ifirst = 0;
-                S.clow = 0.0 + one * S.dc;   // cb(k) is still 0 in mode 1
-                S.c1 = S.c1 - onea * S.dc;
-                S.omega = twopi / S.t1;
-                S.wvno = S.omega / S.c1;
-                S.ph = RootSearch::kGsFirst;
-                return true;
-            }
-            cg[S.k - 1] = (float)S.ck;
-        } else {
-            const float cc0 = (float)S.ck;
-            const float ccg = (float)S.c1;
-            cg[S.k - 1] = (1.0f / S.t1a - 1.0f / S.t1b) / (1.0f / (S.t1a * cc0) - 1.0f / (S.t1b * ccg));
-        }
-        S.cprev = S.ck;
-        S.ph = RootSearch::kStart;
-        continue;
-    getsol_fail:
-        if (S.stage == 0) {   // the fundamental mode fails from this period on
-            for (int i = S.k; i <= S.kmax; i++) cg[i - 1] = 0.0;
-            S.ph = RootSearch::kDone;
-            S.status = 1;
-            return false;
-        }
-        {   // the second search failed: the group velocity uses c itself
-            const float cc0 = (float)S.ck;
-            const float ccg = (float)S.ck;
-            cg[S.k - 1] = (1.0f / S.t1a - 1.0f / S.t1b) / (1.0f / (S.t1a * cc0) - 1.0f / (S.t1b * ccg));
-        }
-        S.cprev = S.ck;
-        S.ph = RootSearch::kStart;
-    }
-}
-
-// surfdisp96() with the searches of all lanes meeting at one dltar call
-// (see RootSearch); same arguments and results, mode 1.
-static __device__ int surfdisp96_lockstep(const LayerConst& L, const float* vpm, const float* vsm,
-                                          const float* rhom, int iflsph, int iwave, int igr,
-                                          int kmax, const double* t, double* cg) {
-    SDModel M;
-    RootSearch S;
-    sd_setup(L, vpm, vsm, rhom, iflsph, iwave, M, S.betmx, S.cc, S.dc);
-    const int ifunc = (iwave == 1) ? 1 : 2;
-    S.cm = S.cc;
-    S.igr = igr;
-    S.kmax = kmax;
-    S.ph = RootSearch::kStart;
-    S.k = 0;
-    S.status = 0;
-    S.cprev = 0.0;
-    S.ck = 0.0;
-    double del = 0.0;
-    while (root_advance(S, M, del, t, cg)) del = dltar(M, S.wvno, S.omega, ifunc);
-    return S.status;
+    first_velocity(L.mmax, vmin, M.a, M.b, betmx, cc, dc);
 }
 
 // ---------------------------------------------------------------------------
@@ -1334,11 +852,8 @@ __device__ __forceinline__ double normc_ex(double* ee, int nmat) {
     for (int i = 0; i < nmat; i++)
         if (fabs(ee[i]) > t1) t1 = fabs(ee[i]);
     if (t1 < 1.e-40) t1 = 1.0;
-    for (int i = 0; i < nmat; i++) {
-        double t2 = ee[i];
-        t2 = t2 / t1;
-        ee[i] = t2;
-    }
+    const double rh = 1.0 / t1, rl = recip_lo(t1, rh);
+    for (int i = 0; i < nmat; i++) ee[i] = quot(ee[i], t1, rh, rl);
     return sk_log(t1);
 }
 
