@@ -303,8 +303,7 @@ __device__ __forceinline__ double fwd_solve(const BatchArgs<S>& B, const SrcInfo
     P.nx = nx;
     P.ny = ny;
     if constexpr (sizeof(S) == sizeof(double)) {
-        P.dx = g.dx;
-        P.dy = g.dy;
+        P.h = make_spacing64(g.dx, g.dy);
     } else {
         P.idx = (float)(1.0 / g.dx);
         P.idy = (float)(1.0 / g.dy);
