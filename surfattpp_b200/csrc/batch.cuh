@@ -85,10 +85,11 @@ __host__ __device__ inline SlotLayout slot_layout(int nx, int ny, int maxr) {
     L.Ta = take(n * sizeof(S));
     L.sadj = take(r * sizeof(double));
     L.syn = take(r * sizeof(double));
-    L.flags = take(n);   // per-cell sweep flags of the FP64 forward (systolic.cuh)
+    // which neighbours a cell's winning stencil reads (discrete_adjoint)
+    L.flags = take(sizeof(S) == sizeof(double) ? n : 0);
     // per-row x ranges (systolic.cuh): [0, ny) cells that can change in the
     // current sweep, [ny, 2 ny) cells changed in the current iteration,
-    // [2 ny, 3 ny) the adjoint's ranges for the next sweep
+    // [2 ny, 3 ny) the ranges for the next sweep
     L.rng = take(3 * (size_t)ny * sizeof(int2));
     // tail teams (systolic.cuh, Team): per strip its record and the last
     // sweep's L1 partials of its 32 lanes
@@ -290,7 +291,7 @@ __device__ __forceinline__ void team_serve(BlockTeams* bt) {
 template <class S, bool ISO, int VAR>
 __device__ __forceinline__ double fwd_solve(const BatchArgs<S>& B, const SrcInfo& si, int ip,
                                             int src, S* tau, S* tst, Q4<S>* pk,
-                                            unsigned char* flags, int2* rng, double* T,
+                                            int2* rng, double* T,
                                             int& iters, int& status, BlockTeams* bt) {
     const Grid& g = B.g;
     const int nx = g.nx, ny = g.ny;
@@ -325,7 +326,6 @@ __device__ __forceinline__ double fwd_solve(const BatchArgs<S>& B, const SrcInfo
     P.b_iso = B.b_iso;
     P.tau = tau;
     P.tau_start = tst;
-    P.flags = flags;
     P.rng = rng;
     P.crng = rng + ny;
     P.rng2 = rng + 2 * ny;
@@ -352,7 +352,6 @@ __device__ __forceinline__ double fwd_solve(const BatchArgs<S>& B, const SrcInfo
         const S v = (fixed ? S(1) : S(10)) - off;
         tau[k] = v;
         tst[k] = v;
-        if (Pol::kFlags) flags[k] = 1;
     });
     for (int iy = lane; iy < ny; iy += 32) {
         rng[iy] = make_int2(0, nx - 1);
@@ -705,7 +704,6 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
     double* P_sadj = reinterpret_cast<double*>(base + L.sadj);
     double* P_syn = reinterpret_cast<double*>(base + L.syn);
     Q4<S>* P_pk = reinterpret_cast<Q4<S>*>(base + L.PK);
-    unsigned char* P_fl = base + L.flags;
     int2* P_rng = reinterpret_cast<int2*>(base + L.rng);
     {
         const int ip = B.ev.iper[e];
@@ -717,8 +715,8 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
 
         if (B.mode != MODE_ADJ_ONLY) {
             int iters = 0;
-            fwd_solve<S, ISO, VAR>(B, si, ip, B.ev.src[e], P_tau, P_tst, P_pk, P_fl, P_rng,
-                                   P_T, iters, status, bt);
+            fwd_solve<S, ISO, VAR>(B, si, ip, B.ev.src[e], P_tau, P_tst, P_pk, P_rng, P_T, iters,
+                                   status, bt);
             if (lane == 0 && B.out.fwd_iters) B.out.fwd_iters[e] = iters;
             if (B.out.T_out)
                 for (size_t k = lane; k < n; k += 32) B.out.T_out[(size_t)e * n + k] = P_T[k];

@@ -37,29 +37,21 @@ struct Nb {
 // neighbour values and the cell's own data only (the forward keeps
 // min(current, candidates), the adjoint recomputes from its neighbours), so a
 // cell none of whose neighbours changed since its last update would come out
-// bit-identical: the sweep skips it.  This is exact -- fields, iteration
-// counts and convergence sums are the same as updating every cell.
-// Per cell a flag byte records
-//   bit 0: a neighbour changed after the cell's last visit (update it next),
-//   bit 1: the cell's value changed at its last visit.
-// At its visit a cell is dirty if bit 0 is set or its left or upper
-// neighbour (visited just before it in this sweep) changed.  The flags of a
-// visited cell are written one step later, when its right neighbour (this
-// lane) and lower neighbour (next lane) have been visited.  The strip's first
-// lane reads bit 1 of the row above (previous strip) and sets bit 0 there when
-// it changes.  A warp step whose 32 cells are all clean skips the update math.
-// All flags start at 1 (every cell is updated at its first visit).
+// bit-identical: rows are marched only over the columns that can change (see
+// "Marching only where something can change" below).  This is exact --
+// fields, iteration counts and convergence sums are the same as updating
+// every cell.
 //
-// P must provide: types V (field value), X (neighbour aux), Cell {V v; X x;
-//   unsigned fl;}, kLead, nrows(), ncols(), stride() (row pitch), row(rp, yd),
-//   col(cp, xd) (sweep-ordered -> grid index), begin_row(iy, active),
-//   load(k, last) -> Cell and load_nb(k) -> Cell (v, x, fl) at grid offset k,
+// P must provide: types V (field value), X (neighbour aux), Cell {V v; X x;},
+//   kLead, nrows(), ncols(), stride() (row pitch), row(rp, yd), col(cp, xd)
+//   (sweep-ordered -> grid index), begin_row(iy, active), load(k, last) ->
+//   Cell and load_nb(k) -> Cell (v, x) at grid offset k,
 //   update(cur, ix, xm, xp, ym, yp, xd, yd) -> V with xm / ym the upwind and
 //   xp / yp the downwind neighbours in sweep order, account(cur, v, l1, linf)
 //   (last sweep of an iteration), store(k, v, write_v, write_start),
-//   store_flag(k, f), cp_of(ix, xd) (grid x -> sweep-ordered column, the
-//   inverse of col), rng and crng (per-row x ranges of flag bit 0 and of
-//   cells changed in the current iteration, see below).
+//   cp_of(ix, xd) (grid x -> sweep-ordered column, the inverse of col), rng,
+//   rng2 and crng (per-row x ranges of cells that can change in this sweep
+//   and in the next one, and of cells changed in this iteration, see below).
 template <class V>
 __device__ __forceinline__ bool same_bits(V a, V b);
 template <>
@@ -156,11 +148,7 @@ struct March {
     V prev_v;           // this lane's previous result (upwind-x of its next cell)
     X prev_x;
     unsigned bal;       // ballot of "changed" of the previous step
-    unsigned pfl;       // flags of this lane's previous cell
-    int rmin, rmax;     // grid x range of this row's cells left with bit 0 set
-    int umin, umax;     // lane 0: grid x where its row changed (bit 0 set above)
     int cmin, cmax;     // grid x range of this row's cells changed in this march
-    int uf, ul;         // sweep columns where the row above changed in this sweep
     int lf, ll;         // sweep columns where the strip's last row changed
 };
 
@@ -198,25 +186,12 @@ __device__ __forceinline__ void systolic_step(P& p, March<V, X>& L, const int t,
         dn_v = ecur.v;
         dn_x = ecur.x;
     }
-    bool work = true;
-    if constexpr (P::kFlags) {
-        // left neighbour changed: own bit of the last ballot; upper: lane-1's
-        // bit (the strip's first lane reads bit 1 of the row above, current
-        // only where that row changed in this sweep)
-        unsigned up_chg = lane > 0 ? (L.bal >> (lane - 1)) & 1u : 0u;
-        if (L.eup) up_chg = (c >= L.uf && c <= L.ul) ? (ecur.fl >> 1) & 1u : 0u;
-        const bool dirty = valid && (((cur.fl | (L.bal >> lane) | up_chg) & 1u) != 0u);
-        work = __any_sync(FULL_MASK, dirty);
-    }
     bool chg = false;
-    int ix = 0;
     if (valid) {
-        ix = p.col(c, xd);
-        V nv = cur.v;
-        if (work)
-            nv = p.update(cur, ix, Nb<V, X>{c > 0, L.prev_v, L.prev_x},
-                          Nb<V, X>{c + 1 < NC, nx1.v, nx1.x}, Nb<V, X>{L.has_up, up_v, up_x},
-                          Nb<V, X>{L.has_dn, dn_v, dn_x}, xd, L.yd);
+        const int ix = p.col(c, xd);
+        const V nv = p.update(cur, ix, Nb<V, X>{c > 0, L.prev_v, L.prev_x},
+                              Nb<V, X>{c + 1 < NC, nx1.v, nx1.x}, Nb<V, X>{L.has_up, up_v, up_x},
+                              Nb<V, X>{L.has_dn, dn_v, dn_x}, xd, L.yd);
         chg = !same_bits(nv, cur.v);
         bool wst = false;
         if (L.last) {
@@ -232,26 +207,6 @@ __device__ __forceinline__ void systolic_step(P& p, March<V, X>& L, const int t,
         L.prev_x = cur.x;
     }
     const unsigned nbal = __ballot_sync(FULL_MASK, chg);
-    // flags of the previous cell (r', c-1): changed at its visit; a later
-    // neighbour (right = this cell, lower = lane+1's cell of this step) changed
-    if constexpr (P::kFlags) {
-        if (L.act && c >= 1 && c <= NC) {
-            const int ixp = p.col(c - 1, xd);
-            const unsigned lower = (lane + 1 < L.nr_strip) ? (nbal >> (lane + 1)) & 1u : 0u;
-            const unsigned f = (((L.bal >> lane) & 1u) << 1) | ((nbal >> lane) & 1u) | lower;
-            if (f != L.pfl) p.store_flag(L.ioff + ixp, f);
-            if (f & 1u) {
-                L.rmin = min(L.rmin, ixp);
-                L.rmax = max(L.rmax, ixp);
-            }
-        }
-        if (L.eup && chg) {
-            p.store_flag(L.eoff + ix, ecur.fl | 1u);
-            L.umin = min(L.umin, ix);
-            L.umax = max(L.umax, ix);
-        }
-        if (valid) L.pfl = cur.fl;
-    }
     if ((nbal >> (L.nr_strip - 1)) & 1u) {
         const int cl = t - (L.nr_strip - 1);
         L.lf = min(L.lf, cl);
@@ -260,12 +215,15 @@ __device__ __forceinline__ void systolic_step(P& p, March<V, X>& L, const int t,
     L.bal = nbal;
 }
 
-// Marching only where something can change.  Per row the policy keeps the
-// grid x range of its cells with flag bit 0 set (p.rng[iy], empty when
-// x > y).  A strip's cells can only change from column `first` on: the
-// first column of its rows' ranges, or where the row above changed in this
-// sweep.  Before it every cell is clean and stays so, so the march starts
-// there: each lane takes its previous cell (value, aux, flags) from memory
+// Marching only where something can change.  A cell can only change in a
+// sweep if one of its four neighbours changed since its last visit, so per
+// row the policy keeps the grid x range of such cells: p.rng[iy] (empty when
+// x > y), the union of the previous sweep's changed ranges of rows iy-1, iy,
+// iy+1 widened by one column (collected in p.rng2, swapped in at the end of
+// the sweep; every cell that could change in a sweep is visited in it).  A
+// strip's cells can only change from column `first` on: the first column of
+// its rows' ranges, or where the row above changed in this sweep.  The march
+// starts there: each lane takes its previous cell (value, aux) from memory
 // and the pipeline is filled from that column.  After `lastd` (the last such
 // column) and one step in which no cell changed, nothing can change any
 // more: the march stops.  A strip with nothing to do is not marched.
@@ -275,15 +233,9 @@ __device__ __forceinline__ void systolic_step(P& p, March<V, X>& L, const int t,
 // start-of-iteration copy; every other cell adds an exact zero.  All of
 // this is exact: the cells not visited are exactly those the full march
 // would have left bit-identical and whose sums terms are zero.
-//
-// Without flags (P::kFlags false: short updates, where the per-cell
-// bookkeeping costs more than the updates it saves) every cell of the march
-// is updated, and the ranges come from changes instead: a cell can only
-// change in the next sweep if one of its four neighbours changed in this one
-// (every cell that could change in this sweep was visited in it), so the
-// next sweep's range of row r is the union of this sweep's changed ranges of
-// rows r-1, r, r+1 widened by one column (p.rng2, swapped in at the end of
-// the sweep).
+// Per-cell flags instead (a byte per cell: a neighbour changed since; a warp
+// step of 32 clean cells skips its updates) cost more than they save: 10 %
+// on the FP64 forward sweeps, 14 % on the FP32 ones.
 //
 // P::kLead = how many steps ahead a lane loads its row (1 for the long
 // forward update, more for the short adjoint update).
@@ -313,8 +265,7 @@ __device__ __forceinline__ void systolic_sweep(P& p, const int xd, const int yd,
         // strip 0 follows the previous sweep's last strip; once that one is
         // done the whole sweep is, and next sweep's ranges can be cleared
         if (sweep > 0 && (nstrip - 1) % W != 0) team_wait(*tm, (nstrip - 1) % W, id0 - 1, kStripDone);
-        if constexpr (!P::kFlags)
-            for (int iy = lane; iy < p.ny; iy += 32) p.rng2[iy] = make_int2(0x7fffffff, -1);
+        for (int iy = lane; iy < p.ny; iy += 32) p.rng2[iy] = make_int2(0x7fffffff, -1);
         __threadfence();
         __syncwarp();
     }
@@ -428,18 +379,11 @@ __device__ __forceinline__ void systolic_sweep(P& p, const int xd, const int yd,
         L.edn = lane == nr_strip - 1 && L.has_dn;
         const int iy_up = L.eup ? p.row(rp - 1, yd) : 0;
         L.eoff = L.eup ? iy_up * S : (L.edn ? p.row(rp + 1, yd) * S : 0);
-        L.uf = uf;
-        L.ul = ul;
         L.lf = NC;
         L.ll = -1;
-        L.rmin = 0x7fffffff;
-        L.rmax = -1;
-        L.umin = 0x7fffffff;
-        L.umax = -1;
         L.cmin = 0x7fffffff;
         L.cmax = -1;
         L.bal = 0u;
-        L.pfl = 0u;
         L.prev_v = V(0);
         L.prev_x = X(0);
         p.begin_row(iy, act);
@@ -452,7 +396,6 @@ __device__ __forceinline__ void systolic_sweep(P& p, const int xd, const int yd,
             const Cell q = p.load_nb(L.ioff + p.col(c0 - 1, xd));
             L.prev_v = q.v;
             L.prev_x = q.x;
-            L.pfl = q.fl;
         }
         need(first + LEAD);
         Cell buf[NB], eb[NB];
@@ -468,9 +411,7 @@ __device__ __forceinline__ void systolic_sweep(P& p, const int xd, const int yd,
                 if (L.eup || L.edn) eb[q] = p.load_nb(L.eoff + ixq);
             }
         }
-        // one step more than the march: the last cell's flags are written
-        // one step after its visit
-        const int nsteps = NC + nr_strip;
+        const int nsteps = NC + nr_strip - 1;
         const bool pub = coop && lane == nr_strip - 1;   // publishes the last row's progress
         if constexpr (P::kRolled && LEAD == 1) {
             // one copy of the step (long updates: instruction-cache footprint
@@ -509,7 +450,7 @@ __device__ __forceinline__ void systolic_sweep(P& p, const int xd, const int yd,
                 if (known && t + NB - 1 - 31 > lastd && L.bal == 0u) break;
             }
         }
-        if constexpr (!P::kFlags) {
+        {
             // next sweep's ranges: this row's changes widened by a column, in
             // this row and the rows above and below (a team's neighbouring
             // strips merge into the same rows: atomics)
@@ -546,12 +487,9 @@ __device__ __forceinline__ void systolic_sweep(P& p, const int xd, const int yd,
             // the rows outside the strip
             if (any && (L.eup || L.edn)) merge(L.eup ? iy_up : p.row(rp + 1, yd), lo, hi);
         }
-        // every cell of the row that had bit 0 set was visited: the range is
-        // replaced; lane 0 then adds where it set bit 0 in the row above.
-        // Cells changed since the iteration began: added to, or (after the
-        // last sweep, whose copy makes start == current) cleared.
+        // cells changed since the iteration began: added to, or (after the
+        // last sweep, whose copy makes start == current) cleared
         if (act) {
-            if constexpr (P::kFlags) p.rng[iy] = make_int2(L.rmin, L.rmax);
             if (last) {
                 p.crng[iy] = make_int2(0x7fffffff, -1);
             } else if (L.cmin <= L.cmax) {
@@ -562,12 +500,6 @@ __device__ __forceinline__ void systolic_sweep(P& p, const int xd, const int yd,
             }
         }
         __syncwarp();
-        if (P::kFlags && L.eup && L.umin <= L.umax) {
-            int2 r = p.rng[iy_up];
-            r.x = min(r.x, L.umin);
-            r.y = max(r.y, L.umax);
-            p.rng[iy_up] = r;
-        }
         if constexpr (P::kCoop) {
             if (!coop) l1 += l1s;
             else if (last) tm->sums[j * 32 + lane] = l1s;
@@ -588,15 +520,13 @@ __device__ __forceinline__ void systolic_sweep(P& p, const int xd, const int yd,
         ul = L.ll;
         __syncwarp();
     }
-    if constexpr (!P::kFlags) {
-        int2* nxt = p.rng2;
-        p.rng2 = p.rng;
-        p.rng = nxt;
-        // (a team clears them at the next sweep's start, after this sweep)
-        if (!coop) {
-            for (int iy = lane; iy < p.ny; iy += 32) p.rng2[iy] = make_int2(0x7fffffff, -1);
-            __syncwarp();
-        }
+    int2* nxt = p.rng2;
+    p.rng2 = p.rng;
+    p.rng = nxt;
+    // (a team clears them at the next sweep's start, after this sweep)
+    if (!coop) {
+        for (int iy = lane; iy < p.ny; iy += 32) p.rng2[iy] = make_int2(0x7fffffff, -1);
+        __syncwarp();
     }
 }
 
