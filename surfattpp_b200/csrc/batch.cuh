@@ -12,6 +12,7 @@
 #include "fsm.cuh"
 #include "launch.h"
 
+#include <algorithm>
 #include <type_traits>
 
 // Resident 128-thread blocks per SM the register allocation is sized for.
@@ -288,15 +289,15 @@ __device__ __forceinline__ void team_serve(BlockTeams* bt) {
     }
 }
 
-template <class S, bool ISO, int VAR>
-__device__ __forceinline__ double fwd_solve(const BatchArgs<S>& B, const SrcInfo& si, int ip,
+template <class S, bool ISO, int VAR, class Crew>
+__device__ __forceinline__ double fwd_solve(const Crew& crew, const BatchArgs<S>& B, const SrcInfo& si, int ip,
                                             int src, S* tau, S* tst, Q4<S>* pk,
                                             int2* rng, double* T,
                                             int& iters, int& status, BlockTeams* bt) {
     const Grid& g = B.g;
     const int nx = g.nx, ny = g.ny;
     const size_t n = (size_t)nx * ny;
-    const int lane = threadIdx.x & 31;
+    const int rank = crew.rank(), size = crew.size();
     const double fun0_64 = bilinear64(B.fun64 + (size_t)ip * n, nx, si.idx0, si.idy0, si.r1, si.r2);
     using Pol = typename std::conditional<sizeof(S) == sizeof(double), FwdPolicy64<ISO>,
                                           FwdPolicyDelta32<ISO, variant_fwd_rolled(VAR)>>::type;
@@ -317,7 +318,7 @@ __device__ __forceinline__ double fwd_solve(const BatchArgs<S>& B, const SrcInfo
         const S* Gx = B.Gx + (size_t)src * n;
         const S* Gy = B.Gy + (size_t)src * n;
         const S* fn = B.fun + (size_t)ip * n;
-        for (size_t k = lane; k < n; k += 32)
+        for (size_t k = rank; k < n; k += size)
             st4(pk + k, G[k] * fun0, Gx[k] * fun0, Gy[k] * fun0, fn[k]);
     }
     P.pk = pk;
@@ -334,7 +335,7 @@ __device__ __forceinline__ double fwd_solve(const BatchArgs<S>& B, const SrcInfo
     // rows with |(yy - y0)/dy| <= 1 (src/eikonal_solver.cpp:118-129, :162):
     // one contiguous range, yy being monotone
     int fy0 = ny, fy1 = -1;
-    for (int iy = lane; iy < ny; iy += 32)
+    for (int iy = threadIdx.x & 31; iy < ny; iy += 32)   // (each warp by itself)
         if (fabs((g.yy[iy] - si.y0) / g.dy) <= 1.0) {
             fy0 = min(fy0, iy);
             fy1 = max(fy1, iy);
@@ -347,18 +348,18 @@ __device__ __forceinline__ double fwd_solve(const BatchArgs<S>& B, const SrcInfo
     P.fy1 = fy1;
     // initial tau (src/eikonal_solver.cpp:118-129); FP32 stores u = tau - 1
     const S off = (sizeof(S) == sizeof(double)) ? S(0) : S(1);
-    for_cells(nx, n, lane, [&](size_t k, int ix, int iy) {
+    for_cells(nx, n, rank, size, [&](size_t k, int ix, int iy) {
         const bool fixed = iy >= fy0 && iy <= fy1 && ix >= si.fix_x0 && ix <= si.fix_x1;
         const S v = (fixed ? S(1) : S(10)) - off;
         tau[k] = v;
         tst[k] = v;
     });
-    for (int iy = lane; iy < ny; iy += 32) {
+    for (int iy = rank; iy < ny; iy += size) {
         rng[iy] = make_int2(0, nx - 1);
         rng[ny + iy] = make_int2(0x7fffffff, -1);   // crng: nothing changed yet
         rng[2 * ny + iy] = make_int2(0x7fffffff, -1);
     }
-    __syncwarp();
+    crew.sync();
     iters = 0;
     // stopping rule: the reference's (src/eikonal_solver.cpp:292-303), or,
     // for the exact discrete adjoint, a fixed point (an iteration in which
@@ -367,7 +368,7 @@ __device__ __forceinline__ double fwd_solve(const BatchArgs<S>& B, const SrcInfo
     unsigned helpers = 0;   // tail team (FP32 variants with teams)
     for (int iter = 0; iter < 2000; iter++) {
         double l1 = 0.0, linf = 0.0;
-        if constexpr (variant_teams(VAR) && sizeof(S) == sizeof(float)) {
+        if constexpr (!Crew::kWide && variant_teams(VAR) && sizeof(S) == sizeof(float)) {
             // (alone: the sweeps of the variants without teams, the same code)
             const Team tm = bt ? team_begin(bt, helpers, 0, P, ny)
                                : Team{1, 0, nullptr, nullptr, nullptr, nullptr};
@@ -379,16 +380,15 @@ __device__ __forceinline__ double fwd_solve(const BatchArgs<S>& B, const SrcInfo
                     systolic_sweep(P, sweep_xd(sw), sweep_yd(sw), sw == 3, l1, linf);
             }
         } else {
-            for (int sw = 0; sw < 4; sw++)
-                systolic_sweep(P, sweep_xd(sw), sweep_yd(sw), sw == 3, l1, linf);
+            for (int sw = 0; sw < 4; sw++) crew.sweep(P, sw, l1, linf);
         }
         iters = iter + 1;
-        const double L1 = warp_sum(l1) / (double)(nx * ny);
-        const double Linf = warp_max(linf);
+        const double L1 = crew.sum(l1) / (double)(nx * ny);
+        const double Linf = crew.max(linf);
         if (B.discrete ? (Linf == 0.0) : (L1 < 1e-4 && Linf < 1e-4)) break;
         if (iter == 1999) status = ST_NOCONV;
     }
-    if constexpr (variant_teams(VAR) && sizeof(S) == sizeof(float)) {
+    if constexpr (!Crew::kWide && variant_teams(VAR) && sizeof(S) == sizeof(float)) {
         if (bt) {
             team_release(bt, helpers);
             if (__shfl_sync(FULL_MASK, *(volatile int*)&bt->err, 0)) status = ST_TEAM;
@@ -397,15 +397,15 @@ __device__ __forceinline__ double fwd_solve(const BatchArgs<S>& B, const SrcInfo
     // T = tau * T0 in FP64 (src/eikonal_solver.cpp:317)
     const double* G64 = B.G64 + (size_t)src * n;
     bool finite = true;
-    for (size_t k = lane; k < n; k += 32) {
+    for (size_t k = rank; k < n; k += size) {
         const double t0 = G64[k] * fun0_64;
         const double t = (sizeof(S) == sizeof(double)) ? (double)tau[k] * t0
                                                          : t0 + (double)tau[k] * t0;
         T[k] = t;
         if (!isfinite(t)) finite = false;
     }
-    if (!__all_sync(FULL_MASK, finite)) status = ST_NONFINITE;
-    __syncwarp();
+    if (!crew.all(finite)) status = ST_NONFINITE;
+    crew.sync();
     return fun0_64;
 }
 
@@ -519,14 +519,14 @@ __device__ inline WinD discrete_winner(const double* tau, const Q4<double>* pk, 
     return best;
 }
 
-template <bool ISO>
-__device__ inline void discrete_adjoint(const BatchArgs<double>& B, unsigned int e,
+template <bool ISO, class Crew>
+__device__ inline void discrete_adjoint(const Crew& crew, const BatchArgs<double>& B, unsigned int e,
                                         unsigned char* base, const SrcInfo& si, int ip, int nr,
                                         int& status) {
     const Grid& g = B.g;
     const int nx = g.nx, ny = g.ny;
     const size_t n = (size_t)nx * ny;
-    const int lane = threadIdx.x & 31;
+    const int rank = crew.rank(), size = crew.size();
     const SlotLayout L = slot_layout<double>(nx, ny, B.maxr);
     double* tau = reinterpret_cast<double*>(base + L.tau);
     double* tst = reinterpret_cast<double*>(base + L.tst);
@@ -546,7 +546,7 @@ __device__ inline void discrete_adjoint(const BatchArgs<double>& B, unsigned int
     const int r0 = B.ev.rec_ptr[e];
     // fixed source cells (src/eikonal_solver.cpp:118-129)
     int fy0 = ny, fy1 = -1;
-    for (int iy = lane; iy < ny; iy += 32)
+    for (int iy = threadIdx.x & 31; iy < ny; iy += 32)   // (each warp by itself)
         if (fabs((g.yy[iy] - si.y0) / g.dy) <= 1.0) {
             fy0 = min(fy0, iy);
             fy1 = max(fy1, iy);
@@ -556,7 +556,7 @@ __device__ inline void discrete_adjoint(const BatchArgs<double>& B, unsigned int
         fy1 = max(fy1, __shfl_xor_sync(FULL_MASK, fy1, o));
     }
     // 1. the winning stencils and their partials
-    for_cells(nx, n, lane, [&](size_t k, int ix, int iy) {
+    for_cells(nx, n, rank, size, [&](size_t k, int ix, int iy) {
         const bool fixed = iy >= fy0 && iy <= fy1 && ix >= si.fix_x0 && ix <= si.fix_x1;
         WinD w{};
         w.ok = false;
@@ -578,11 +578,11 @@ __device__ inline void discrete_adjoint(const BatchArgs<double>& B, unsigned int
             DD[k] = make_double2(0.0, 0.0);
         }
     });
-    __syncwarp();
+    crew.sync();
     // 2. the receivers' explicit fun0 term, then the adjoint source g in the
     // tau plane (tau is no longer needed)
     double srec = 0.0;
-    if (lane == 0)
+    if (rank == 0)
         for (int ir = 0; ir < nr; ir++) {
             const double d = sadj[ir];
             const int st = B.ev.rec_idx[r0 + ir];
@@ -593,11 +593,11 @@ __device__ inline void discrete_adjoint(const BatchArgs<double>& B, unsigned int
                 continue;
             for (int q = 0; q < 4; q++) srec += d * wq[q] * tau[kq[q]] * G[kq[q]];
         }
-    srec = __shfl_sync(FULL_MASK, srec, 0);
-    __syncwarp();
-    for (size_t k = lane; k < n; k += 32) tau[k] = 0.0;
-    __syncwarp();
-    if (lane == 0)
+    srec = crew.first(srec);
+    crew.sync();
+    for (size_t k = rank; k < n; k += size) tau[k] = 0.0;
+    crew.sync();
+    if (rank == 0)
         for (int ir = 0; ir < nr; ir++) {
             const double d = sadj[ir];
             const int st = B.ev.rec_idx[r0 + ir];
@@ -608,10 +608,10 @@ __device__ inline void discrete_adjoint(const BatchArgs<double>& B, unsigned int
                 continue;
             for (int q = 0; q < 4; q++) tau[kq[q]] += d * wq[q] * PK[kq[q]].x;
         }
-    __syncwarp();
+    crew.sync();
     // 3. the sweep weights at every cell: the partials of the neighbours'
     // winners that read this cell
-    for_cells(nx, n, lane, [&](size_t k, int ix, int iy) {
+    for_cells(nx, n, rank, size, [&](size_t k, int ix, int iy) {
         const double wxm = (ix > 0 && (fl[k - 1] & 3u) == 2u) ? Jx[k - 1] : 0.0;
         const double wxp = (ix < nx - 1 && (fl[k + 1] & 3u) == 1u) ? Jx[k + 1] : 0.0;
         const double wym = (iy > 0 && ((fl[k - nx] >> 2) & 3u) == 2u) ? Jy[k - nx] : 0.0;
@@ -620,12 +620,12 @@ __device__ inline void discrete_adjoint(const BatchArgs<double>& B, unsigned int
         lam[k] = 0.0;
         tst[k] = 0.0;
     });
-    for (int iy = lane; iy < ny; iy += 32) {
+    for (int iy = rank; iy < ny; iy += size) {
         rng[iy] = make_int2(0, nx - 1);
         rng[ny + iy] = make_int2(0x7fffffff, -1);
         rng[2 * ny + iy] = make_int2(0x7fffffff, -1);
     }
-    __syncwarp();
+    crew.sync();
     // 4. lambda to its fixed point
     AdjPolicyLinear64 Q;
     Q.nx = nx;
@@ -640,19 +640,19 @@ __device__ inline void discrete_adjoint(const BatchArgs<double>& B, unsigned int
     int iters = 0;
     for (int iter = 0; iter < 2000; iter++) {
         double l1 = 0.0, linf = 0.0;
-        for (int sw = 0; sw < 4; sw++) systolic_sweep(Q, sweep_xd(sw), sweep_yd(sw), sw == 3, l1, linf);
+        for (int sw = 0; sw < 4; sw++) crew.sweep(Q, sw, l1, linf);
         iters = iter + 1;
-        if (warp_max(linf) == 0.0) break;
+        if (crew.max(linf) == 0.0) break;
         if (iter == 1999) status = ST_NOCONV;
     }
-    if (lane == 0 && B.out.adj_iters) B.out.adj_iters[e] = iters;
+    if (rank == 0 && B.out.adj_iters) B.out.adj_iters[e] = iters;
     // 5. dchi/dsvel = -dchi/dfun fun^2
     const double* fun = B.fun64 + (size_t)ip * n;
     double* acc = B.out.adj_s ? B.out.adj_s + (size_t)ip * n : nullptr;
     double* con = B.out.contrib ? B.out.contrib + (size_t)(e - B.out.contrib_e0) * n : nullptr;
     double s0 = 0.0;
     bool finite = true;
-    for (size_t k = lane; k < n; k += 32) {
+    for (size_t k = rank; k < n; k += size) {
         const double lk = lam[k];
         s0 += lk * DD[k].y;
         const double gf = (fl[k] & 16u) ? lk * DD[k].x : 0.0;
@@ -661,9 +661,9 @@ __device__ inline void discrete_adjoint(const BatchArgs<double>& B, unsigned int
         if (con) con[k] = v;
         else if (acc && v != 0.0) atomicAdd(acc + k, v);
     }
-    const double S = srec + warp_sum(s0);
-    __syncwarp();
-    if (lane == 0) {
+    const double S = srec + crew.sum(s0);
+    crew.sync();
+    if (rank == 0) {
         const int i0 = si.idx0, j0 = si.idy0;
         const size_t kk[4] = {(size_t)j0 * nx + i0, (size_t)(j0 + 1) * nx + i0,
                               (size_t)j0 * nx + i0 + 1, (size_t)(j0 + 1) * nx + i0 + 1};
@@ -676,10 +676,10 @@ __device__ inline void discrete_adjoint(const BatchArgs<double>& B, unsigned int
             else if (acc && v != 0.0) atomicAdd(acc + kk[q], v);
         }
     }
-    if (!__all_sync(FULL_MASK, finite)) status = ST_NONFINITE;
+    if (!crew.all(finite)) status = ST_NONFINITE;
     // the delta plane is zero between events
-    for (size_t k = lane; k < n; k += 32) Jy[k] = 0.0;
-    __syncwarp();
+    for (size_t k = rank; k < n; k += size) Jy[k] = 0.0;
+    crew.sync();
 }
 
 // One event of the batch on the warp's scratch slot `base` (laid out for
@@ -688,11 +688,11 @@ __device__ inline void discrete_adjoint(const BatchArgs<double>& B, unsigned int
 // `clear_delta`: the slot last held an event of another grid size, whose
 // planes overlap this grid's adjoint-source plane, so it is zeroed first (in
 // a single-grid launch it is zero between events by construction).
-template <class S, bool ISO, int VAR>
-__device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int e,
+template <class S, bool ISO, int VAR, class Crew>
+__device__ __forceinline__ void batch_event(const Crew& crew, const BatchArgs<S>& B, unsigned int e,
                                             unsigned char* base, bool clear_delta = false,
                                             BlockTeams* bt = nullptr) {
-    const int lane = threadIdx.x & 31;
+    const int rank = crew.rank(), size = crew.size();
     const Grid& g = B.g;
     const int nx = g.nx, ny = g.ny;
     const size_t n = (size_t)nx * ny;
@@ -715,13 +715,13 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
 
         if (B.mode != MODE_ADJ_ONLY) {
             int iters = 0;
-            fwd_solve<S, ISO, VAR>(B, si, ip, B.ev.src[e], P_tau, P_tst, P_pk, P_rng, P_T, iters,
+            fwd_solve<S, ISO, VAR>(crew, B, si, ip, B.ev.src[e], P_tau, P_tst, P_pk, P_rng, P_T, iters,
                                    status, bt);
-            if (lane == 0 && B.out.fwd_iters) B.out.fwd_iters[e] = iters;
+            if (rank == 0 && B.out.fwd_iters) B.out.fwd_iters[e] = iters;
             if (B.out.T_out)
-                for (size_t k = lane; k < n; k += 32) B.out.T_out[(size_t)e * n + k] = P_T[k];
+                for (size_t k = rank; k < n; k += size) B.out.T_out[(size_t)e * n + k] = P_T[k];
             // synthetic times at the receivers (src/preproc.cpp:105-115)
-            for (int ir = lane; ir < nr; ir += 32) {
+            for (int ir = rank; ir < nr; ir += size) {
                 const int st = B.ev.rec_idx[r0 + ir];
                 const double ts =
                     interp2d_pt(g.xx_deg, nx, g.yy_deg, ny, P_T, B.ev.stlo[st], B.ev.stla[st]);
@@ -735,8 +735,8 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
                                  ? 0.0
                                  : B.ev.weight[r0 + ir] * (ts - B.ev.tt_obs[r0 + ir]);
             }
-            __syncwarp();
-            if (B.mode == MODE_FWD_ADJ && lane == 0 && B.out.chi_ev) {
+            crew.sync();
+            if (B.mode == MODE_FWD_ADJ && rank == 0 && B.out.chi_ev) {
                 double s = 0.0;   // src/preproc.cpp:142, receivers in order
                 for (int ir = 0; ir < nr; ir++) {
                     const double r = P_syn[ir] - B.ev.tt_obs[r0 + ir];
@@ -746,8 +746,8 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
             }
         } else {
             T = B.ev.T_in + (size_t)e * n;
-            for (int ir = lane; ir < nr; ir += 32) P_sadj[ir] = B.ev.sadj[r0 + ir];
-            __syncwarp();
+            for (int ir = rank; ir < nr; ir += size) P_sadj[ir] = B.ev.sadj[r0 + ir];
+            crew.sync();
         }
 
         // pass 0: the adjoint of the residuals (or the given source); pass 1
@@ -757,7 +757,7 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
         bool discrete = false;
         if constexpr (sizeof(S) == sizeof(double)) {
             if (B.discrete && B.mode == MODE_FWD_ADJ) {
-                discrete_adjoint<ISO>(B, e, base, si, ip, nr, status);
+                discrete_adjoint<ISO>(crew, B, e, base, si, ip, nr, status);
                 discrete = true;
             }
         }
@@ -765,17 +765,17 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
                           : (B.mode == MODE_FWD_ADJ && B.out.kden_s && !B.ev.sadj) ? 2
                                                                                    : 1;
         if (clear_delta && npass > 0) {
-            for (size_t k = lane; k < n; k += 32) P_delta[k] = 0.0;
-            __syncwarp();
+            for (size_t k = rank; k < n; k += size) P_delta[k] = 0.0;
+            crew.sync();
         }
         for (int pass = 0; pass < npass; pass++) {
             if (pass == 1) {
-                for (int ir = lane; ir < nr; ir += 32) P_sadj[ir] = -B.ev.weight[r0 + ir] * 1.0;
-                __syncwarp();
+                for (int ir = rank; ir < nr; ir += size) P_sadj[ir] = -B.ev.weight[r0 + ir] * 1.0;
+                crew.sync();
             }
             // adjoint source (src/eikonal_solver.cpp:354-375), receivers in order
-            if (lane == 0) spread_delta(g, B.ev, r0, nr, P_sadj, P_delta, false);
-            __syncwarp();
+            if (rank == 0) spread_delta(g, B.ev, r0, nr, P_sadj, P_delta, false);
+            crew.sync();
             const double* a_a = ISO ? nullptr : B.a_a64 + (size_t)ip * n;
             const double* b_p = ISO ? nullptr : B.b_p64 + (size_t)ip * n;
             const double* c_a = ISO ? nullptr : B.c_a64 + (size_t)ip * n;
@@ -796,7 +796,7 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
                 double* P_Tst = reinterpret_cast<double*>(P_tst);
                 // face fluxes (src/eikonal_solver.cpp:404-441): a2(ix) is a1(ix+1)
                 // and b2(iy) is b1(iy+1), identical expressions in the reference
-                for_cells(nx, n, lane, [&](size_t k, int ix, int iy) {
+                for_cells(nx, n, rank, size, [&](size_t k, int ix, int iy) {
                     const bool interior = ix >= 1 && ix <= nx - 2 && iy >= 1 && iy <= ny - 2;
                     double a1p = 0, a2m = 0, b1p = 0, b2m = 0, d = 0;
                     if (interior) {
@@ -818,12 +818,12 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
                     P_Ta[k] = v0;
                     P_Tst[k] = v0;
                 });
-                for (int iy = lane; iy < ny; iy += 32) {
+                for (int iy = rank; iy < ny; iy += size) {
                     P_rng[iy] = make_int2(1, nx - 2);
                     P_rng[ny + iy] = make_int2(0x7fffffff, -1);
                     P_rng[2 * ny + iy] = make_int2(0x7fffffff, -1);
                 }
-                __syncwarp();
+                crew.sync();
                 AdjPolicyExact Q;
                 Q.nx = nx;
                 Q.ny = ny;
@@ -839,11 +839,10 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
                 if (big)
                     for (int iter = 0; iter < 1000; iter++) {
                         double l1 = 0.0, linf = 0.0;
-                        for (int sw = 0; sw < 4; sw++)
-                            systolic_sweep(Q, sweep_xd(sw), sweep_yd(sw), sw == 3, l1, linf);
+                        for (int sw = 0; sw < 4; sw++) crew.sweep(Q, sw, l1, linf);
                         iters = iter + 1;
-                        const double L1 = warp_sum(l1) / (double)(nx * ny);
-                        const double Linf = warp_max(linf);
+                        const double L1 = crew.sum(l1) / (double)(nx * ny);
+                        const double Linf = crew.max(linf);
                         if (L1 < 1e-9 && Linf < 1e-9) break;
                     }
             } else {
@@ -871,7 +870,7 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
                     return -(T[k] - T[k - nx]) * idy * bv
                            + (T[k + 1] - T[k - 1] + T[k + 1 - nx] - T[k - 1 - nx]) * i4dx * cv;
                 };
-                for_cells(nx, n, lane, [&](size_t k, int ix, int iy) {
+                for_cells(nx, n, rank, size, [&](size_t k, int ix, int iy) {
                     const bool interior = ix >= 1 && ix <= nx - 2 && iy >= 1 && iy <= ny - 2;
                     float c0 = 0.f, wxm = 0.f, wxp = 0.f, wym = 0.f, wyp = 0.f;
                     if (interior) {
@@ -897,12 +896,12 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
                     P_Ta[k] = v0;
                     P_tst[k] = v0;
                 });
-                for (int iy = lane; iy < ny; iy += 32) {
+                for (int iy = rank; iy < ny; iy += size) {
                     P_rng[iy] = make_int2(1, nx - 2);
                     P_rng[ny + iy] = make_int2(0x7fffffff, -1);
                     P_rng[2 * ny + iy] = make_int2(0x7fffffff, -1);
                 }
-                __syncwarp();
+                crew.sync();
                 AdjPolicyW32<variant_adj_lead(VAR)> Q;
                 Q.nx = nx;
                 Q.ny = ny;
@@ -917,7 +916,7 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
                 if (big)
                     for (int iter = 0; iter < 1000; iter++) {
                         double l1 = 0.0, linf = 0.0;
-                        if constexpr (variant_teams(VAR)) {
+                        if constexpr (!Crew::kWide && variant_teams(VAR)) {
                             const Team tm = bt ? team_begin(bt, helpers, 1, Q, ny)
                                                : Team{1, 0, nullptr, nullptr, nullptr, nullptr};
                             if (tm.W > 1) {
@@ -931,49 +930,48 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
                                                    linf);
                             }
                         } else {
-                            for (int sw = 0; sw < 4; sw++)
-                                systolic_sweep(Q, sweep_xd(sw), sweep_yd(sw), sw == 3, l1, linf);
+                            for (int sw = 0; sw < 4; sw++) crew.sweep(Q, sw, l1, linf);
                         }
                         iters = iter + 1;
-                        const double L1 = warp_sum(l1) / (double)(nx * ny);
-                        const double Linf = warp_max(linf);
+                        const double L1 = crew.sum(l1) / (double)(nx * ny);
+                        const double Linf = crew.max(linf);
                         if (L1 < 1e-9 && Linf < 1e-9) break;
                         // FP32 fixed point: no cell changed by more than a few
                         // ulps of the field's largest magnitude
                         float vm = 0.f;
                         const float4* T4 = reinterpret_cast<const float4*>(P_Ta);
-                        for (size_t k = lane; k < n / 4; k += 32) {
+                        for (size_t k = rank; k < n / 4; k += size) {
                             const float4 q = T4[k];
                             vm = fmaxf(vm, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)),
                                                  fmaxf(fabsf(q.z), fabsf(q.w))));
                         }
-                        for (size_t k = (n / 4) * 4 + lane; k < n; k += 32)
+                        for (size_t k = (n / 4) * 4 + rank; k < n; k += size)
                             vm = fmaxf(vm, fabsf(P_Ta[k]));
-                        const double vmax = warp_max((double)vm);
+                        const double vmax = crew.max((double)vm);
                         if (Linf <= 4.0 * 5.960464477539063e-08 * vmax) break;
                     }
-                if constexpr (variant_teams(VAR)) {
+                if constexpr (!Crew::kWide && variant_teams(VAR)) {
                     if (bt) {
                         team_release(bt, helpers);
                         if (__shfl_sync(FULL_MASK, *(volatile int*)&bt->err, 0)) status = ST_TEAM;
                     }
                 }
             }
-            if (lane == 0 && B.out.adj_iters && pass == 0) B.out.adj_iters[e] = iters;
-            if (lane == 0) spread_delta(g, B.ev, r0, nr, P_sadj, P_delta, true);
+            if (rank == 0 && B.out.adj_iters && pass == 0) B.out.adj_iters[e] = iters;
+            if (rank == 0) spread_delta(g, B.ev, r0, nr, P_sadj, P_delta, true);
             bool finite = true;
             const S* TaS = reinterpret_cast<const S*>(base + L.Ta);
             if (pass == 1) {
                 const double* inv3 = B.inv3 + (size_t)ip * n;
                 double* acc = B.out.kden_s + (size_t)ip * n;
-                for (size_t k = lane; k < n; k += 32) {
+                for (size_t k = rank; k < n; k += size) {
                     const double v = (double)TaS[k];
                     if (!isfinite(v)) finite = false;
                     const double c = v * inv3[k];
                     if (c != 0.0) atomicAdd(acc + k, c);
                 }
             } else if (B.mode == MODE_ADJ_ONLY) {
-                for (size_t k = lane; k < n; k += 32) {
+                for (size_t k = rank; k < n; k += size) {
                     const double v = (double)TaS[k];
                     if (!isfinite(v)) finite = false;
                     if (B.out.Ta_out) B.out.Ta_out[(size_t)e * n + k] = v;
@@ -986,7 +984,7 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
                 double* con = B.out.contrib
                                   ? B.out.contrib + (size_t)(e - B.out.contrib_e0) * n
                                   : nullptr;
-                for_cells(nx, n, lane, [&](size_t k, int ix, int iy) {
+                for_cells(nx, n, rank, size, [&](size_t k, int ix, int iy) {
                     double v = (double)TaS[k];
                     if (ix >= mb.ix_lo && ix <= mb.ix_hi && iy >= mb.iy_lo && iy <= mb.iy_hi) v = 0.0;
                     if (!isfinite(v)) finite = false;
@@ -996,11 +994,11 @@ __device__ __forceinline__ void batch_event(const BatchArgs<S>& B, unsigned int 
                     else if (acc && c != 0.0) atomicAdd(acc + k, c);
                 });
             }
-            if (!__all_sync(FULL_MASK, finite)) status = ST_NONFINITE;
-            __syncwarp();
+            if (!crew.all(finite)) status = ST_NONFINITE;
+            crew.sync();
         }
-        if (lane == 0 && B.out.status) B.out.status[e] = status;
-        __syncwarp();
+        if (rank == 0 && B.out.status) B.out.status[e] = status;
+        crew.sync();
     }
 }
 
@@ -1034,7 +1032,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs<S>& B) {
                 const unsigned int qi = warp_next_event(B.sc.queue);
                 if (qi >= (unsigned)B.ev.ne) break;
                 const unsigned int e = B.sc.order ? (unsigned)B.sc.order[qi] : qi;
-                batch_event<S, ISO, VAR>(B, e, base, false, &bt);
+                batch_event<S, ISO, VAR>(WarpCrew{}, B, e, base, false, &bt);
             }
             if ((threadIdx.x & 31) == 0) atomicSub(&bt.busy, 1);
         }
@@ -1047,7 +1045,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs<S>& B) {
             const unsigned int qi = warp_next_event(B.sc.queue);
             if (qi >= (unsigned)B.ev.ne) break;
             const unsigned int e = B.sc.order ? (unsigned)B.sc.order[qi] : qi;
-            batch_event<S, ISO, VAR>(B, e, base);
+            batch_event<S, ISO, VAR>(WarpCrew{}, B, e, base);
         }
     }
 }
@@ -1056,6 +1054,29 @@ template <class S, bool ISO, int VAR>
 __global__ void __launch_bounds__(128, sizeof(S) == sizeof(double) ? SA_MINB64 : SA_MINB32)
 batch_kernel(BatchArgs<S> B) {
     batch_body<S, ISO, VAR>(B);
+}
+
+// The same for solves too few to fill the GPU with a warp each: a block per
+// scratch slot and event (wide_sweep).  MAXT bounds the block size.
+template <class S, bool ISO, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB)
+batch_wide_kernel(BatchArgs<S> B, const double* __restrict__ dxdy) {
+    __shared__ WideShared sh;
+    if (dxdy) {   // the grid spacing in device memory
+        B.g.dx = dxdy[0];
+        B.g.dy = dxdy[1];
+    }
+    const BlockCrew crew{&sh};
+    unsigned char* base = B.sc.base + (size_t)blockIdx.x * B.sc.slot_bytes;
+    for (;;) {
+        if (threadIdx.x == 0) sh.next = atomicAdd(B.sc.queue, 1u);
+        __syncthreads();
+        const unsigned int qi = sh.next;
+        if (qi >= (unsigned)B.ev.ne) break;
+        const unsigned int e = B.sc.order ? (unsigned)B.sc.order[qi] : qi;
+        batch_event<S, ISO, 0>(crew, B, e, base);
+        __syncthreads();
+    }
 }
 
 // One persistent launch over the events of several plans (grid levels of
@@ -1074,7 +1095,7 @@ batch_multi_kernel(const BatchArgs<S>* __restrict__ levels, unsigned int ntotal,
         const unsigned int qi = warp_next_event(sc.queue);
         if (qi >= ntotal) break;
         const unsigned int c = code[qi];
-        batch_event<S, ISO, VAR>(levels[c >> 24], c & 0xffffffu, base, true);
+        batch_event<S, ISO, VAR>(WarpCrew{}, levels[c >> 24], c & 0xffffffu, base, true);
     }
 }
 
@@ -1137,6 +1158,49 @@ inline BatchArgs<float> make_batch_args<float>(const BatchDesc& d) {
     B.mode = d.mode;
     B.discrete = d.discrete;
     return B;
+}
+
+// Warps per event of a launch (1: batch_kernel, a warp each): as many as give
+// an SM `load` warps together, at most one per 32 rows and `most`, evened out
+// over the strips.
+inline int wide_warps(const BatchDesc& d, int load, int most) {
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const int strips = (d.g.ny + 31) / 32;
+    const long long fit = (long long)load * nsm / std::max(d.ev.ne, 1);
+    const int W = (int)std::min<long long>(std::min(fit, (long long)most), strips);
+    if (W <= 1) return 1;
+    const int turns = (strips + W - 1) / W;
+    return (strips + turns - 1) / turns;
+}
+
+// Launches batch_wide_kernel where several warps per event are the faster
+// (always with dxdy); false: the caller launches batch_kernel.  With 10 warps
+// an SM (FP64) no measured size is slower than with a warp each: 61 / 101 /
+// 201 / 301 rows x 300 events 6.0 -> 5.4, 14.7 -> 9.3, 69 -> 40, 94 -> 51 ms;
+// x 600 events 6.1 -> 5.5, 15.4 -> 12.5, 68 -> 54, 93 -> 71; x 1000 events
+// (one warp) 7.1, 16.6, 69.  The shorter FP32 steps pay more for the barrier
+// between them, the more the fewer rows a sweep has: with 14 / 10 / 4 warps
+// an SM from 161 / 65 / fewer rows, 301 rows x 300 / 1000 events 50 -> 27, 56
+// -> 53 ms; 101 rows x 300 / 740 6.8 -> 5.6, 8.5 -> 8.2; 61 rows x 300 / 450
+// 2.68 -> 2.65, 2.73 -> 3.15 (not taken).
+template <class S, int BIG>
+inline bool launch_wide(const BatchDesc& d, const double* dxdy, cudaStream_t st) {
+    const int load = sizeof(S) == sizeof(double) ? 10 : d.g.ny > 160 ? 14 : d.g.ny > 64 ? 10 : 4;
+    const int W = wide_warps(d, load, BIG / 32);
+    if (W <= 1 && !dxdy) return false;
+    const BatchArgs<S> B = make_batch_args<S>(d);
+    const int blocks = std::max(1, std::min(d.sc.nslots, d.ev.ne));
+    constexpr int MINB = sizeof(S) == sizeof(double) ? SA_MINB64 : SA_MINB32;
+    if (W <= 4) {
+        if (d.iso) batch_wide_kernel<S, true, 128, MINB><<<blocks, 32 * W, 0, st>>>(B, dxdy);
+        else batch_wide_kernel<S, false, 128, MINB><<<blocks, 32 * W, 0, st>>>(B, dxdy);
+    } else {
+        if (d.iso) batch_wide_kernel<S, true, BIG, 1><<<blocks, 32 * W, 0, st>>>(B, dxdy);
+        else batch_wide_kernel<S, false, BIG, 1><<<blocks, 32 * W, 0, st>>>(B, dxdy);
+    }
+    return true;
 }
 
 }  // namespace sa

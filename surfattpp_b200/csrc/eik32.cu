@@ -50,6 +50,7 @@ void launch_variant(const BatchDesc& d, const BatchArgs<float>& B, int blocks, c
 }  // namespace
 
 cudaError_t launch_batch32(const BatchDesc& d, cudaStream_t st) {
+    if (d.variant == 0 && launch_wide<float, 512>(d, nullptr, st)) return cudaGetLastError();
     const BatchArgs<float> B = make_batch_args<float>(d);
     // with tail teams every resident warp runs (the slots in use are spread
     // over the blocks, the other warps start as helpers)

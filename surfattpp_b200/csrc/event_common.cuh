@@ -189,15 +189,15 @@ __device__ inline MaskBox mask_box(const Grid& g, double x0, double y0) {
     return m;
 }
 
-// Per-lane walk over the cells of an nx-wide plane of n cells in warp
-// stride: f(k, ix, iy) at k = lane, lane + 32, ...  The column and row are
-// carried along instead of divided out of k (a 64-bit division per cell).
+// Walk of one of `size` threads over the cells of an nx-wide plane of n cells:
+// f(k, ix, iy) at k = rank, rank + size, ...  The column and row are carried
+// along instead of divided out of k (a 64-bit division per cell).
 template <class F>
-__device__ __forceinline__ void for_cells(int nx, size_t n, int lane, F&& f) {
-    int ix = lane % nx, iy = lane / nx;
-    for (size_t k = lane; k < n; k += 32) {
+__device__ __forceinline__ void for_cells(int nx, size_t n, int rank, int size, F&& f) {
+    int ix = rank % nx, iy = rank / nx;
+    for (size_t k = rank; k < n; k += size) {
         f(k, ix, iy);
-        ix += 32;
+        ix += size;
         while (ix >= nx) {
             ix -= nx;
             iy++;

@@ -530,6 +530,253 @@ __device__ __forceinline__ void systolic_sweep(P& p, const int xd, const int yd,
     }
 }
 
+// ---------------------------------------------------------------------------
+// The same sweep by a whole block, for solves too few to fill the GPU with a
+// warp each: a strip is as many rows as the block has threads (up to 512), a
+// row per thread, one anti-diagonal step between two block barriers, so a
+// sweep takes NC + NR steps instead of
+// (NR / 32) (NC + 32).  A warp's first lane takes its upper neighbour (the
+// last lane of the warp above) through shared memory; its last lane streams
+// the old values of the row below from memory as a strip's last lane does:
+// the row's owner reaches a column two steps after its last reader has
+// consumed it.  Cell updates, ranges and skipping are those of
+// systolic_sweep.  Bound by the instructions of a warp's step, of which an SM
+// now holds several at a time: 16 FP64 solves and adjoints of 301x301 80.4 ms
+// with a warp each, 52.5 / 39.4 / 33.7 / 29.4 ms with 2 / 4 / 5 / 10 warps
+// (FP32 39 -> 16 ms).  Meeting once in 8 steps instead (each warp 7 steps
+// further behind the one above) gains nothing: 29.3 ms, and 3.2 instead of
+// 2.9 ms on 250 solves of 41x41.
+// ---------------------------------------------------------------------------
+constexpr int kWideWarps = 16;
+struct WideShared {
+    double2 up[2][kWideWarps];     // by step parity: last lane's value and aux
+    int red[2][kWideWarps];
+    double dred[kWideWarps];
+    int uf, ul;                    // columns where the strip's last row changed
+    double bcast;
+    unsigned next;
+};
+
+// One step of a thread at column c; up: what the warp above left (its first
+// lane, below the strip's first row) or null, out: what this warp leaves (its
+// last lane) or null.
+template <int LEAD, class P, class Cell, class V, class X>
+__device__ __forceinline__ bool wide_step(P& p, March<V, X>& L, const int c, Cell& cur, Cell& nx1,
+                                          Cell& ld, Cell& ecur, Cell& eld, double& l1,
+                                          double& linf, const double2* up, double2* out) {
+    const int NC = L.NC, xd = L.xd;
+    const bool valid = L.act && (unsigned)c < (unsigned)NC;
+    const int c2 = c + 1 + LEAD;
+    if (L.act && (unsigned)c2 < (unsigned)NC) {
+        const int ix2 = p.col(c2, xd);
+        ld = p.load(L.ioff + ix2, L.last);
+        if (L.eup || L.edn) eld = p.load_nb(L.eoff + ix2);
+    }
+    V up_v = __shfl_up_sync(FULL_MASK, L.prev_v, 1);
+    X up_x = __shfl_up_sync(FULL_MASK, L.prev_x, 1);
+    V dn_v = __shfl_down_sync(FULL_MASK, nx1.v, 1);
+    X dn_x = __shfl_down_sync(FULL_MASK, nx1.x, 1);
+    if (up) {
+        const double2 u = *up;
+        up_v = (V)u.x;
+        up_x = (X)u.y;
+    }
+    if (L.eup) {
+        up_v = ecur.v;
+        up_x = ecur.x;
+    }
+    if (L.edn) {
+        dn_v = ecur.v;
+        dn_x = ecur.x;
+    }
+    bool chg = false;
+    if (valid) {
+        const int ix = p.col(c, xd);
+        const V nv = p.update(cur, ix, Nb<V, X>{c > 0, L.prev_v, L.prev_x},
+                              Nb<V, X>{c + 1 < NC, nx1.v, nx1.x}, Nb<V, X>{L.has_up, up_v, up_x},
+                              Nb<V, X>{L.has_dn, dn_v, dn_x}, xd, L.yd);
+        chg = !same_bits(nv, cur.v);
+        bool wst = false;
+        if (L.last) {
+            p.account(cur, nv, l1, linf);
+            wst = !same_bits(nv, cur.vs);
+        }
+        if (chg || wst) p.store(L.ioff + ix, nv, chg, wst);
+        if (chg) {
+            L.cmin = min(L.cmin, ix);
+            L.cmax = max(L.cmax, ix);
+        }
+        L.prev_v = nv;
+        L.prev_x = cur.x;
+    }
+    if (out) *out = make_double2((double)L.prev_v, (double)L.prev_x);
+    return chg;
+}
+
+template <class P>
+__device__ __forceinline__ void wide_sweep(P& p, const int xd, const int yd, const bool last,
+                                           double& l1, double& linf, WideShared* sh) {
+    using V = typename P::V;
+    using X = typename P::X;
+    using Cell = typename P::Cell;
+    constexpr int LEAD = P::kLead;
+    constexpr int NB = LEAD + 2;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int T = blockDim.x, W = T >> 5;
+    const int NR = p.nrows();
+    const int NC = p.ncols();
+    const int S = p.stride();
+    int uf = NC, ul = -1;
+    for (int k0 = 0; k0 < NR; k0 += T) {
+        const int rp = k0 + tid;
+        const bool act = rp < NR;
+        const int nr_strip = min(T, NR - k0);
+        const int iy = act ? p.row(rp, yd) : 0;
+        int fc = NC, lc = -1;
+        if (act) {   // (ranges are merged by atomics, performed in L2)
+            int2 r = __ldcg(p.rng + iy);
+            if (last) {
+                const int2 q = __ldcg(p.crng + iy);
+                r.x = min(r.x, q.x);
+                r.y = max(r.y, q.y);
+            }
+            if (r.x <= r.y) {
+                const int a = p.cp_of(r.x, xd), b = p.cp_of(r.y, xd);
+                fc = min(a, b);
+                lc = max(a, b);
+            }
+        }
+        fc = __reduce_min_sync(FULL_MASK, fc);
+        lc = __reduce_max_sync(FULL_MASK, lc);
+        if (lane == 0) {
+            sh->red[0][w] = fc;
+            sh->red[1][w] = lc;
+        }
+        __syncthreads();
+        int first = uf, lastd = ul;
+        for (int i = 0; i < W; i++) {
+            first = min(first, sh->red[0][i]);
+            lastd = max(lastd, sh->red[1][i]);
+        }
+        if (first >= NC) {   // no cell of the strip can change
+            uf = NC;
+            ul = -1;
+            __syncthreads();   // red is read before it is written again
+            continue;
+        }
+        March<V, X> L;
+        L.lane = lane;
+        L.NC = NC;
+        L.xd = xd;
+        L.yd = yd;
+        L.last = last;
+        L.act = act;
+        L.nr_strip = nr_strip;
+        L.ioff = iy * S;
+        L.has_up = act && rp > 0;
+        L.has_dn = act && rp + 1 < NR;
+        L.eup = tid == 0 && L.has_up;
+        L.edn = (lane == 31 || tid == nr_strip - 1) && L.has_dn;
+        const bool sup = lane == 0 && w > 0;
+        L.eoff = L.eup ? p.row(rp - 1, yd) * S : (L.edn ? p.row(rp + 1, yd) * S : 0);
+        L.cmin = 0x7fffffff;
+        L.cmax = -1;
+        L.prev_v = V(0);
+        L.prev_x = X(0);
+        p.begin_row(iy, act);
+        const int c0 = first - tid;   // column at step t: t - tid
+        if (act && c0 >= 1) {
+            const Cell q = p.load_nb(L.ioff + p.col(c0 - 1, xd));
+            L.prev_v = q.v;
+            L.prev_x = q.x;
+        }
+        if (lane == 31) sh->up[(first - 1) & 1][w] = make_double2((double)L.prev_v, (double)L.prev_x);
+        Cell buf[NB], eb[NB];
+#pragma unroll
+        for (int q = 0; q < NB; q++) {
+            buf[q] = Cell{};
+            eb[q] = Cell{};
+            const int cq = c0 + q;
+            if (q <= LEAD && act && cq >= 0 && cq < NC) {
+                const int ixq = p.col(cq, xd);
+                buf[q] = p.load(L.ioff + ixq, last);
+                if (L.eup || L.edn) eb[q] = p.load_nb(L.eoff + ixq);
+            }
+        }
+        __syncthreads();
+        const int nsteps = NC + nr_strip - 1;
+        const int tail = lastd + nr_strip - 1;   // a step beyond may be the last
+        auto up = [&](int t) { return sup ? &sh->up[(t - 1) & 1][w - 1] : nullptr; };
+        auto out = [&](int t) { return lane == 31 ? &sh->up[t & 1][w] : nullptr; };
+        bool more = true;
+        auto meet = [&](int t, bool chg) {
+            if (t <= tail) __syncthreads();
+            else more = __syncthreads_or(chg) != 0;
+        };
+        if constexpr (P::kRolled && LEAD == 1) {
+            Cell cur = buf[0], nx1 = buf[1], ecur = eb[0], enx1 = eb[1];
+            for (int t = first; more && t < nsteps; t++) {
+                Cell ld = cur, eld = ecur;
+                const bool chg = wide_step<LEAD>(p, L, t - tid, cur, nx1, ld, ecur, eld, l1, linf,
+                                                 up(t), out(t));
+                cur = nx1;
+                nx1 = ld;
+                ecur = enx1;
+                enx1 = eld;
+                meet(t, chg);
+            }
+        } else {
+            for (int t = first; more && t < nsteps; t += NB) {
+#pragma unroll
+                for (int i = 0; i < NB; i++) {
+                    if (more && t + i < nsteps)
+                        meet(t + i, wide_step<LEAD>(p, L, t + i - tid, buf[i % NB],
+                                                    buf[(i + 1) % NB], buf[(i + 1 + LEAD) % NB],
+                                                    eb[i % NB], eb[(i + 1 + LEAD) % NB], l1, linf,
+                                                    up(t + i), out(t + i)));
+                }
+            }
+        }
+        // next sweep's ranges, and the cells changed in this iteration
+        const bool any = L.cmin <= L.cmax;
+        if (any) {
+            const int lo = max(L.cmin - 1, p.col(0, 1)), hi = min(L.cmax + 1, p.col(NC - 1, 1));
+            auto merge = [&](int row) {
+                int* q = reinterpret_cast<int*>(p.rng2 + row);
+                atomicMin(q, lo);
+                atomicMax(q + 1, hi);
+            };
+            merge(iy);
+            if (L.has_up) merge(p.row(rp - 1, yd));
+            if (L.has_dn) merge(p.row(rp + 1, yd));
+        }
+        if (act) {
+            if (last) {
+                p.crng[iy] = make_int2(0x7fffffff, -1);
+            } else if (any) {
+                int2 q = __ldcg(p.crng + iy);
+                q.x = min(q.x, L.cmin);
+                q.y = max(q.y, L.cmax);
+                p.crng[iy] = q;
+            }
+        }
+        if (tid == nr_strip - 1) {
+            const int a = any ? p.cp_of(L.cmin, xd) : NC, b = any ? p.cp_of(L.cmax, xd) : -1;
+            sh->uf = any ? min(a, b) : NC;
+            sh->ul = any ? max(a, b) : -1;
+        }
+        __syncthreads();
+        uf = sh->uf;
+        ul = sh->ul;
+    }
+    int2* nxt = p.rng2;
+    p.rng2 = p.rng;
+    p.rng = nxt;
+    __syncthreads();
+    for (int iy = tid; iy < p.ny; iy += T) p.rng2[iy] = make_int2(0x7fffffff, -1);
+    __syncthreads();
+}
+
 // The four sweep directions of src/eikonal_solver.cpp:137-140 (and :466-469).
 __device__ __forceinline__ int sweep_xd(int s) { return s < 2 ? 1 : -1; }
 __device__ __forceinline__ int sweep_yd(int s) { return (s & 1) ? -1 : 1; }
@@ -542,5 +789,61 @@ __device__ __forceinline__ double warp_max(double v) {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(FULL_MASK, v, o));
     return v;
 }
+
+// Who works on one event: a warp or a block.  rank / size number its threads,
+// sum and max leave the result in every thread.
+struct WarpCrew {
+    static constexpr bool kWide = false;
+    __device__ __forceinline__ int rank() const { return threadIdx.x & 31; }
+    __device__ __forceinline__ int size() const { return 32; }
+    __device__ __forceinline__ void sync() const { __syncwarp(); }
+    __device__ __forceinline__ bool all(bool b) const { return __all_sync(FULL_MASK, b); }
+    __device__ __forceinline__ double sum(double v) const { return warp_sum(v); }
+    __device__ __forceinline__ double max(double v) const { return warp_max(v); }
+    __device__ __forceinline__ double first(double v) const {
+        return __shfl_sync(FULL_MASK, v, 0);
+    }
+    template <class P>
+    __device__ __forceinline__ void sweep(P& p, int s, double& l1, double& linf) const {
+        systolic_sweep(p, sweep_xd(s), sweep_yd(s), s == 3, l1, linf);
+    }
+};
+struct BlockCrew {
+    static constexpr bool kWide = true;
+    WideShared* sh;
+    __device__ __forceinline__ int rank() const { return threadIdx.x; }
+    __device__ __forceinline__ int size() const { return blockDim.x; }
+    __device__ __forceinline__ void sync() const { __syncthreads(); }
+    __device__ __forceinline__ bool all(bool b) const { return __syncthreads_and(b) != 0; }
+    __device__ __forceinline__ double sum(double v) const {
+        v = warp_sum(v);
+        if ((threadIdx.x & 31) == 0) sh->dred[threadIdx.x >> 5] = v;
+        __syncthreads();
+        double s = 0.0;
+        for (int i = 0; i < (int)(blockDim.x >> 5); i++) s += sh->dred[i];
+        __syncthreads();
+        return s;
+    }
+    __device__ __forceinline__ double max(double v) const {
+        v = warp_max(v);
+        if ((threadIdx.x & 31) == 0) sh->dred[threadIdx.x >> 5] = v;
+        __syncthreads();
+        double s = sh->dred[0];
+        for (int i = 1; i < (int)(blockDim.x >> 5); i++) s = fmax(s, sh->dred[i]);
+        __syncthreads();
+        return s;
+    }
+    __device__ __forceinline__ double first(double v) const {
+        if (threadIdx.x == 0) sh->bcast = v;
+        __syncthreads();
+        v = sh->bcast;
+        __syncthreads();
+        return v;
+    }
+    template <class P>
+    __device__ __forceinline__ void sweep(P& p, int s, double& l1, double& linf) const {
+        wide_sweep(p, sweep_xd(s), sweep_yd(s), s == 3, l1, linf, sh);
+    }
+};
 
 }  // namespace sa
