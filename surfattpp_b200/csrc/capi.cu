@@ -2104,16 +2104,38 @@ extern "C" int sa_topo_media(sa_ctx* ctx, int nx, int ny, const double* lon, con
     SA_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     const size_t n = (size_t)nx * ny;
-    DArr<double> dlon, dlat, zs;
-    SA_CUDA(dlon.upload(lon, nx, st));
-    SA_CUDA(dlat.upload(lat, ny, st));
-    SA_CUDA(zs.alloc(n));
-    for (int ip = 0; ip < nper; ip++) {
-        // each period starts from the unsmoothed gridded topography (:93-96, :113-114)
-        SA_CUDA(launch_gauss_geo(nx, ny, z_gridded, dlon.p, dlat.p, sigma_deg[ip], zs.p, st));
-        SA_CUDA(launch_topo_media(nx, ny, zs.p, dlon.p, dlat.p, m11 + ip * n, m12 + ip * n,
-                                  m22 + ip * n, angle + ip * n, st));
+    // An evenly spaced longitude grid (up to rounding: 1e-9 of the smallest
+    // sigma) shares a row's weights between its cells; others weigh every
+    // point of every cell.
+    const double h = (lon[nx - 1] - lon[0]) / (nx - 1);
+    const double smin = *std::min_element(sigma_deg, sigma_deg + nper);
+    const double smax = *std::max_element(sigma_deg, sigma_deg + nper);
+    std::vector<double> tables(lon, lon + nx);   // lon, off, lat, sigma
+    double worst = 0.0;
+    for (int m = 0; m < nx; m++) {
+        tables.push_back(std::fma(-(double)m, h, lon[m] - lon[0]));
+        worst = std::max(worst, std::abs(tables.back()));
     }
+    tables.insert(tables.end(), lat, lat + ny);
+    tables.insert(tables.end(), sigma_deg, sigma_deg + nper);
+    // (the window's width in points must be the one lon[1] - lon[0] gives)
+    bool even = h > 0.0 && worst <= 1e-9 * smin && gauss_rows_fits(nx, nper);
+    for (int ip = 0; even && ip < nper; ip++)
+        even = (int)std::min(3.0 * sigma_deg[ip] / h, 1e9) ==
+               (int)std::min(3.0 * sigma_deg[ip] / (lon[1] - lon[0]), 1e9);
+    DArr<double> dtab, zs;
+    SA_CUDA(dtab.upload(tables.data(), tables.size(), st));
+    const double *dlon = dtab.p, *doff = dlon + nx, *dlat = doff + nx, *dsig = dlat + ny;
+    // each period starts from the unsmoothed gridded topography (:93-96, :113-114)
+    SA_CUDA(zs.alloc(n * nper));
+    if (even) {
+        SA_CUDA(launch_gauss_rows(nx, ny, nper, z_gridded, dlat, doff, h, dsig, smax, zs.p, st));
+    } else {
+        for (int ip = 0; ip < nper; ip++)
+            SA_CUDA(launch_gauss_geo(nx, ny, z_gridded, dlon, dlat, sigma_deg[ip], zs.p + ip * n,
+                                     st));
+    }
+    SA_CUDA(launch_topo_media(nx, ny, nper, zs.p, dlon, dlat, m11, m12, m22, angle, st));
     SA_CUDA(cudaStreamSynchronize(st));
     return SA_OK;
 }
