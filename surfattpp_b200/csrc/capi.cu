@@ -83,6 +83,7 @@ struct sa_ctx {
     LayerConstCache lc;
     PeriodCache pc;
     DArr<double> red;   // reduction scratch of the optimizer entry points
+    double* red_host = nullptr;   // and their results (pinned)
     // launch configuration chosen by sa_plan_autotune per grid size:
     // (nx, ny, precision) -> (variant, active slots; 0 = all)
     std::map<std::array<int, 3>, std::array<int, 2>> tune;
@@ -181,6 +182,7 @@ extern "C" void sa_ctx_destroy(sa_ctx* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
+    if (ctx->red_host) cudaFreeHost(ctx->red_host);
     delete ctx;
 }
 
@@ -1831,13 +1833,18 @@ extern "C" int sa_pde_smooth(sa_ctx* ctx, int nx, int ny, int nz, double dx_deg,
 namespace {
 constexpr int LBFGS_STORE = 5;   // MAX_LBFGS_STORE, include/config.h:90
 
-// Reduction helper: runs on `st`, waits, returns the scalar.
-int reduce_to_host(sa_ctx* ctx, cudaError_t launched, double* scratch, double* out,
-                   cudaStream_t st) {
-    SA_CUDA(launched);
-    SA_CUDA(cudaMemcpyAsync(out, scratch + reduce_scratch_doubles() - 1, sizeof(double),
-                            cudaMemcpyDeviceToHost, st));
-    SA_CUDA(cudaStreamSynchronize(st));
+// Reduction scratch and the host words (pinned, device-visible) that the
+// reductions of the optimizer entry points leave their results in.
+int ctx_red(sa_ctx* ctx) {
+    if (!ctx->red.p) {
+        const size_t n = reduce_scratch_doubles();
+        SA_CUDA(ctx->red.alloc(n));
+        SA_CUDA(cudaMemsetAsync(ctx->red.p, 0, n * sizeof(double), ctx->stream));
+        SA_CUDA(cudaStreamSynchronize(ctx->stream));
+    }
+    if (!ctx->red_host)
+        SA_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&ctx->red_host), 4 * sizeof(double),
+                              cudaHostAllocDefault));
     return SA_OK;
 }
 }  // namespace
@@ -1845,10 +1852,12 @@ int reduce_to_host(sa_ctx* ctx, cudaError_t launched, double* scratch, double* o
 struct sa_lbfgs {
     sa_ctx* ctx = nullptr;
     size_t n = 0;
-    // ring of the last LBFGS_STORE + 1 iterates: model (vs) and gradient
+    // ring of the last LBFGS_STORE + 1 iterates: model (vs) and gradient, and
+    // of the pairs (k, k + 1) between them, in iterate k's slot
     DArr<double> model[LBFGS_STORE + 1], grad[LBFGS_STORE + 1];
     int stored_iter[LBFGS_STORE + 1];
-    DArr<double> s[LBFGS_STORE], y[LBFGS_STORE], red;
+    DArr<double> s[LBFGS_STORE + 1], y[LBFGS_STORE + 1], red;
+    DArr<LbfgsScalars> scalars;
 };
 
 extern "C" int sa_lbfgs_create(sa_ctx* ctx, size_t n, sa_lbfgs** out) {
@@ -1859,7 +1868,10 @@ extern "C" int sa_lbfgs_create(sa_ctx* ctx, size_t n, sa_lbfgs** out) {
     L->ctx = ctx;
     L->n = n;
     for (int i = 0; i <= LBFGS_STORE; i++) L->stored_iter[i] = -1;
-    cudaError_t e = L->red.alloc(reduce_scratch_doubles());
+    const size_t nr = reduce_scratch_doubles();
+    cudaError_t e = L->red.alloc(nr);
+    if (e == cudaSuccess) e = L->scalars.alloc(1);
+    if (e == cudaSuccess) e = cudaMemsetAsync(L->red.p, 0, nr * sizeof(double), ctx->stream);
     if (e != cudaSuccess) {
         delete L;
         return fail(ctx, SA_ERR_NOMEM, "sa_lbfgs_create: device allocation failed");
@@ -1879,14 +1891,39 @@ extern "C" int sa_lbfgs_store(sa_lbfgs* L, int iter, const double* model, const 
     sa_ctx* ctx = L->ctx;
     if (iter < 0 || !model || !grad) return fail(ctx, SA_ERR_ARG, "sa_lbfgs_store: arguments");
     SA_CUDA(cudaSetDevice(ctx->device));
-    const int slot = iter % (LBFGS_STORE + 1);
-    SA_CUDA(L->model[slot].alloc(L->n));
-    SA_CUDA(L->grad[slot].alloc(L->n));
-    SA_CUDA(cudaMemcpyAsync(L->model[slot].p, model, L->n * sizeof(double),
-                            cudaMemcpyDeviceToDevice, ctx->stream));
-    SA_CUDA(cudaMemcpyAsync(L->grad[slot].p, grad, L->n * sizeof(double),
-                            cudaMemcpyDeviceToDevice, ctx->stream));
-    SA_CUDA(cudaStreamSynchronize(ctx->stream));
+    static_assert(LBFGS_STORE + 1 == kLbfgsPairs, "pair slots");
+    cudaStream_t st = ctx->stream;
+    const size_t n = L->n;
+    const int R = LBFGS_STORE + 1, slot = iter % R;
+    SA_CUDA(L->model[slot].alloc(n));
+    SA_CUDA(L->grad[slot].alloc(n));
+    L->stored_iter[slot] = -1;
+    // the copy and the pair with the iterate before in one pass; an iterate
+    // stored anew also changes the pair with the one after
+    const int before = iter > 0 && L->stored_iter[(iter - 1) % R] == iter - 1 ? (iter - 1) % R : -1;
+    const int after = L->stored_iter[(iter + 1) % R] == iter + 1 ? (iter + 1) % R : -1;
+    auto pair_slot = [&](int k) { return k % R; };
+    double *s0 = nullptr, *y0 = nullptr;
+    if (before >= 0) {
+        const int p = pair_slot(iter - 1);
+        SA_CUDA(L->s[p].alloc(n));
+        SA_CUDA(L->y[p].alloc(n));
+        s0 = L->s[p].p;
+        y0 = L->y[p].p;
+    }
+    SA_CUDA(launch_lbfgs_store(n, model, grad, L->model[slot].p, L->grad[slot].p,
+                               before >= 0 ? L->model[before].p : nullptr,
+                               before >= 0 ? L->grad[before].p : nullptr, s0, y0, L->red.p,
+                               L->scalars.p, before >= 0 ? pair_slot(iter - 1) : 0, st));
+    if (after >= 0) {
+        const int p = pair_slot(iter);
+        SA_CUDA(L->s[p].alloc(n));
+        SA_CUDA(L->y[p].alloc(n));
+        SA_CUDA(launch_lbfgs_store(n, L->model[after].p, L->grad[after].p, nullptr, nullptr,
+                                   L->model[slot].p, L->grad[slot].p, L->s[p].p, L->y[p].p,
+                                   L->red.p, L->scalars.p, p, st));
+    }
+    SA_CUDA(cudaStreamSynchronize(st));
     L->stored_iter[slot] = iter;
     return SA_OK;
 }
@@ -1904,108 +1941,73 @@ extern "C" int sa_lbfgs_direction(sa_lbfgs* L, int iter, double* dir) {
     SA_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     const size_t n = L->n;
-    auto M = [&](int k) { return L->model[k % (LBFGS_STORE + 1)].p; };
-    auto G = [&](int k) { return L->grad[k % (LBFGS_STORE + 1)].p; };
-    double rho[LBFGS_STORE] = {0}, alpha[LBFGS_STORE] = {0};
-    int rc;
-    for (int h = 0; h < nh; h++) {
-        SA_CUDA(L->s[h].alloc(n));
-        SA_CUDA(L->y[h].alloc(n));
-        SA_CUDA(launch_lbfgs_pair(n, M(h0 + h), M(h0 + h + 1), G(h0 + h), G(h0 + h + 1),
-                                  L->s[h].p, L->y[h].p, st));
-        double sy = 0;
-        if ((rc = reduce_to_host(ctx, launch_dot(n, L->s[h].p, L->y[h].p, L->red.p, st), L->red.p,
-                                 &sy, st)))
-            return rc;
-        rho[h] = (sy > 0.0) ? (1.0 / sy) : 0.0;   // :203
+    const double* g = L->grad[iter % (LBFGS_STORE + 1)].p;
+    if (nh == 0) {
+        SA_CUDA(cudaMemcpyAsync(dir, g, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+        SA_CUDA(cudaStreamSynchronize(st));
+        return SA_OK;
     }
-    // q <- g_iter
-    SA_CUDA(cudaMemcpyAsync(dir, G(iter), n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    for (int h = nh - 1; h >= 0; --h) {   // :209-214
-        double sq = 0;
-        if ((rc = reduce_to_host(ctx, launch_dot(n, L->s[h].p, dir, L->red.p, st), L->red.p, &sq,
-                                 st)))
-            return rc;
-        alpha[h] = rho[h] * sq;
-        SA_CUDA(launch_axpy(n, 0, alpha[h], L->y[h].p, dir, st));
-    }
-    if (nh > 0) {   // :219-228
-        double yy = 0, sy = 0;
-        const int last = nh - 1;
-        if ((rc = reduce_to_host(ctx, launch_dot(n, L->y[last].p, L->y[last].p, L->red.p, st),
-                                 L->red.p, &yy, st)))
-            return rc;
-        if ((rc = reduce_to_host(ctx, launch_dot(n, L->s[last].p, L->y[last].p, L->red.p, st),
-                                 L->red.p, &sy, st)))
-            return rc;
-        const double gamma = (sy > 0.0 && yy > 0.0) ? (sy / yy) : 1.0;
-        SA_CUDA(launch_axpy(n, 1, gamma, nullptr, dir, st));
-    }
-    for (int h = 0; h < nh; ++h) {   // :231-236
-        double yr = 0;
-        if ((rc = reduce_to_host(ctx, launch_dot(n, L->y[h].p, dir, L->red.p, st), L->red.p, &yr,
-                                 st)))
-            return rc;
-        const double beta = rho[h] * yr;
-        SA_CUDA(launch_axpy(n, 2, alpha[h] - beta, L->s[h].p, dir, st));
-    }
+    auto P = [&](int h) { return (h0 + h) % (LBFGS_STORE + 1); };
+    auto S = [&](int h) { return L->s[P(h)].p; };
+    auto Y = [&](int h) { return L->y[P(h)].p; };
+    auto pass = [&](int kind, const double* from, const double* x, const double* d, int slot,
+                    int next) {
+        return launch_lbfgs_pass(n, kind, from, x, d, dir, L->red.p, L->scalars.p, slot, next, st);
+    };
+    // q <- g_iter; the first loop (:209-214), the scaling (:219-228) with its
+    // last pass, the second loop (:231-236)
+    SA_CUDA(pass(0, g, nullptr, S(nh - 1), 0, P(nh - 1)));
+    for (int h = nh - 1; h >= 1; --h)
+        SA_CUDA(pass(1, h == nh - 1 ? g : dir, Y(h), S(h - 1), P(h), P(h - 1)));
+    SA_CUDA(pass(2, nh == 1 ? g : dir, Y(0), Y(0), P(0), P(nh - 1)));
+    for (int h = 0; h + 1 < nh; ++h) SA_CUDA(pass(3, dir, S(h), Y(h + 1), P(h), P(h + 1)));
+    SA_CUDA(pass(4, dir, S(nh - 1), nullptr, P(nh - 1), 0));
     SA_CUDA(cudaStreamSynchronize(st));
     return SA_OK;
 }
 
-namespace {
-double* ctx_red(sa_ctx* ctx, int* rc) {
-    cudaError_t e = ctx->red.alloc(reduce_scratch_doubles());
-    *rc = e == cudaSuccess ? SA_OK : fail(ctx, SA_ERR_NOMEM, "reduction scratch");
-    return ctx->red.p;
-}
-}  // namespace
-
 extern "C" int sa_dot(sa_ctx* ctx, size_t n, const double* a, const double* b, double* out) {
     if (!ctx || !a || !b || !out) return SA_ERR_ARG;
     SA_CUDA(cudaSetDevice(ctx->device));
-    int rc = SA_OK;
-    double* red = ctx_red(ctx, &rc);
+    int rc = ctx_red(ctx);
     if (rc) return rc;
-    return reduce_to_host(ctx, launch_dot(n, a, b, red, ctx->stream), red, out, ctx->stream);
+    SA_CUDA(launch_dot(n, a, b, ctx->red.p, ctx->red_host, ctx->stream));
+    SA_CUDA(cudaStreamSynchronize(ctx->stream));
+    *out = ctx->red_host[0];
+    return SA_OK;
 }
 
 extern "C" int sa_kernel_precondition(sa_ctx* ctx, size_t n, const double* ker_den, double* ker,
                                       void* stream) {
     if (!ctx || !ker_den || !ker) return SA_ERR_ARG;
     SA_CUDA(cudaSetDevice(ctx->device));
-    int rc = SA_OK;
-    double* red = ctx_red(ctx, &rc);
+    int rc = ctx_red(ctx);
     if (rc) return rc;
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-    SA_CUDA(launch_kernel_precondition(n, ker_den, red, ker, st));
+    SA_CUDA(launch_kernel_precondition(n, ker_den, ctx->red.p, ker, st));
     return SA_OK;
 }
 
 extern "C" int sa_grad_normalization(sa_ctx* ctx, size_t n, double* g, double* max_out) {
     if (!ctx || !g) return SA_ERR_ARG;
     SA_CUDA(cudaSetDevice(ctx->device));
-    int rc = SA_OK;
-    double* red = ctx_red(ctx, &rc);
+    int rc = ctx_red(ctx);
     if (rc) return rc;
-    double m = 0;
-    if ((rc = reduce_to_host(ctx, launch_absmax(n, g, red, ctx->stream), red, &m, ctx->stream)))
-        return rc;
-    if (max_out) *max_out = m;
-    if (m < 2.220446049250313e-16) return SA_OK;   // REAL_EPS guard, src/inversion.cpp:316
-    SA_CUDA(launch_axpy(n, 3, m, nullptr, g, ctx->stream));
+    SA_CUDA(launch_normalise(n, g, ctx->red.p, ctx->red_host, ctx->stream));
     SA_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (max_out) *max_out = ctx->red_host[0];
     return SA_OK;
 }
 
 extern "C" int sa_descent_angle(sa_ctx* ctx, size_t n, const double* dir, const double* grad,
                                 double* deg) {
     if (!ctx || !dir || !grad || !deg) return SA_ERR_ARG;
-    double d = 0, gg = 0, dd = 0;
-    int rc;
-    if ((rc = sa_dot(ctx, n, grad, dir, &d))) return rc;
-    if ((rc = sa_dot(ctx, n, grad, grad, &gg))) return rc;
-    if ((rc = sa_dot(ctx, n, dir, dir, &dd))) return rc;
+    SA_CUDA(cudaSetDevice(ctx->device));
+    int rc = ctx_red(ctx);
+    if (rc) return rc;
+    SA_CUDA(launch_dots3(n, grad, dir, ctx->red.p, ctx->red_host, ctx->stream));
+    SA_CUDA(cudaStreamSynchronize(ctx->stream));
+    const double d = ctx->red_host[0], gg = ctx->red_host[1], dd = ctx->red_host[2];
     const double gn = std::sqrt(gg), dn = std::sqrt(dd);   // src/optimize.cpp:46-47
     if (gn < 2.220446049250313e-16 || dn < 2.220446049250313e-16) {
         *deg = 90.0;

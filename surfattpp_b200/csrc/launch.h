@@ -116,18 +116,32 @@ cudaError_t launch_sort_events(int ne, const unsigned int* key_in, unsigned int*
                                cudaStream_t st);
 cudaError_t launch_grad_status(int ncol, const int* colst, const int* ev_worst, int* out,
                                cudaStream_t st);
-// optimize.cu (scratch of reduce_scratch_doubles(); the result lands in its last entry)
+// optimize.cu (scratch of reduce_scratch_doubles(), zeroed once; one
+// reduction at a time).  Results to `out`, device-visible memory.
 size_t reduce_scratch_doubles();
-cudaError_t launch_dot(size_t n, const double* a, const double* b, double* scratch,
+cudaError_t launch_dot(size_t n, const double* a, const double* b, double* scratch, double* out,
                        cudaStream_t st);
-cudaError_t launch_absmax(size_t n, const double* a, double* scratch, cudaStream_t st);
+// out[0..2] = a.b, a.a, b.b
+cudaError_t launch_dots3(size_t n, const double* a, const double* b, double* scratch, double* out,
+                         cudaStream_t st);
+// out = max|g|, then g /= max|g| unless that is below DBL_EPSILON
+cudaError_t launch_normalise(size_t n, double* g, double* scratch, double* out, cudaStream_t st);
 // postproc::kernel_precondition of ker by ker_den (scratch: reduction scratch)
 cudaError_t launch_kernel_precondition(size_t n, const double* ker_den, double* scratch,
                                        double* ker, cudaStream_t st);
-cudaError_t launch_lbfgs_pair(size_t n, const double* m0, const double* m1, const double* g0,
-                              const double* g1, double* s, double* y, cudaStream_t st);
-cudaError_t launch_axpy(size_t n, int kind, double c, const double* x, double* y,
-                        cudaStream_t st);
+// The L-BFGS recursion's scalars by pair slot: s.y, y.y, alpha, alpha - beta.
+// A pair has its first iterate's slot, so that it is valid while both are stored.
+constexpr int kLbfgsPairs = 6;
+struct LbfgsScalars {
+    double sy[kLbfgsPairs], yy[kLbfgsPairs], alpha[kLbfgsPairs], c[kLbfgsPairs];
+};
+cudaError_t launch_lbfgs_store(size_t n, const double* m1, const double* g1, double* m_out,
+                               double* g_out, const double* m0, const double* g0, double* s,
+                               double* y, double* scratch, LbfgsScalars* S, int slot,
+                               cudaStream_t st);
+cudaError_t launch_lbfgs_pass(size_t n, int kind, const double* from, const double* x,
+                              const double* d, double* dir, double* scratch, LbfgsScalars* S,
+                              int slot, int next, cudaStream_t st);
 cudaError_t launch_model_update_vs(size_t n, const double* vs, const double* dir, double alpha,
                                    double* vs_out, double* vp_out, double* rho_out,
                                    cudaStream_t st);
