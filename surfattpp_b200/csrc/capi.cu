@@ -36,13 +36,36 @@ int fail(sa_ctx* ctx, int code, const std::string& msg);
                         std::string(#call) + ": " + cudaGetErrorString(e_));             \
     } while (0)
 
+// Where the arrays of one call come from: a TempScope makes the DArrs that its
+// thread constructs while it lives take their memory from the context's pool,
+// in the order of the call's stream.  The pool keeps at most kPoolKeep bytes
+// between calls and ends with the context.  (cudaMalloc and cudaFree take 10
+// to 100 us each and cudaFree waits for the device: a single solve has 52 of
+// each, 41x41 forward and adjoint 6.4 -> 3.4 ms with the pool.)
+constexpr uint64_t kPoolKeep = 256ull << 20;
+struct TempPool {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t st = nullptr;
+};
+thread_local TempPool t_temp;
+struct TempScope {
+    TempPool before = t_temp;
+    TempScope(sa_ctx* ctx, cudaStream_t st);
+    TempScope(const TempScope&) = delete;
+    ~TempScope() { t_temp = before; }
+};
+
 template <class T>
 struct DArr {
     T* p = nullptr;
     size_t n = 0;
+    const TempPool temp = t_temp;
+    DArr() = default;
+    DArr(const DArr&) = delete;
     ~DArr() { release(); }
     void release() {
-        if (p) cudaFree(p);
+        if (p && temp.pool) cudaFreeAsync(p, temp.st);
+        else if (p) cudaFree(p);
         p = nullptr;
         n = 0;
     }
@@ -50,7 +73,11 @@ struct DArr {
         if (count <= n && p) return cudaSuccess;
         release();
         if (count == 0) count = 1;
-        cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+        void* q = nullptr;
+        cudaError_t e = temp.pool
+                            ? cudaMallocFromPoolAsync(&q, count * sizeof(T), temp.pool, temp.st)
+                            : cudaMalloc(&q, count * sizeof(T));
+        p = static_cast<T*>(q);
         if (e == cudaSuccess) n = count;
         else p = nullptr;
         return e;
@@ -79,6 +106,7 @@ struct PeriodCache {
 struct sa_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaMemPool_t pool = nullptr;   // of the arrays that live for one call
     std::string err;
     LayerConstCache lc;
     PeriodCache pc;
@@ -95,6 +123,8 @@ int fail(sa_ctx* ctx, int code, const std::string& msg) {
     return code;
 }
 
+TempScope::TempScope(sa_ctx* ctx, cudaStream_t st) { t_temp = {ctx->pool, st}; }
+
 struct GraphKey {
     const void* ptr[17];
     int calc_adj;
@@ -110,6 +140,7 @@ struct sa_plan {
     int prec = SA_FP64;
     int nx = 0, ny = 0, nper = 0, ne = 0, nsta = 0, nsrc = 0, npair = 0;
     double dx = 0, dy = 0;
+    std::vector<double> h_xx, h_cosy, h_siny;   // the grid's tables on the host
     DArr<double> xx_deg, yy_deg, xx, yy, cosy, siny, a_f_row64, a_a_row64;
     DArr<float> a_f_row32;
     DArr<double> evlo, evla, stlo, stla, cos_stla;
@@ -174,6 +205,21 @@ extern "C" int sa_ctx_create(int device, sa_ctx** out) {
         delete c;
         return SA_ERR_CUDA;
     }
+    int pools = 0;
+    cudaDeviceGetAttribute(&pools, cudaDevAttrMemoryPoolsSupported, device);
+    if (pools) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        uint64_t keep = kPoolKeep;
+        if (cudaMemPoolCreate(&c->pool, &props) != cudaSuccess) {
+            c->pool = nullptr;
+            cudaGetLastError();
+        } else {
+            cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+    }
     *out = c;
     return SA_OK;
 }
@@ -183,6 +229,7 @@ extern "C" void sa_ctx_destroy(sa_ctx* ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->red_host) cudaFreeHost(ctx->red_host);
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     delete ctx;
 }
 
@@ -212,7 +259,11 @@ int plan_grid(sa_plan* P, const double* xx_deg, const double* yy_deg) {
     sa_ctx* ctx = P->ctx;
     const int nx = P->nx, ny = P->ny;
     cudaStream_t st = ctx->stream;
-    std::vector<double> xr(nx), yr(ny), cy(ny), sy(ny), af(ny), aa(ny);
+    std::vector<double> &xr = P->h_xx, &cy = P->h_cosy, &sy = P->h_siny;
+    xr.resize(nx);
+    cy.resize(ny);
+    sy.resize(ny);
+    std::vector<double> yr(ny), af(ny), aa(ny);
     std::vector<float> af32(ny);
     const double R2 = R_EARTH * R_EARTH;
     for (int i = 0; i < nx; i++) xr[i] = xx_deg[i] * DEG2RAD;
@@ -283,8 +334,7 @@ int plan_events(sa_plan* P, int ne, const double* evlo, const double* evla, cons
     }
     const int nsrc = (int)ux.size();
     P->nsrc = nsrc;
-    std::vector<double> hxx(nx);
-    SA_CUDA(cudaMemcpy(hxx.data(), P->xx.p, nx * sizeof(double), cudaMemcpyDeviceToHost));
+    const std::vector<double>& hxx = P->h_xx;
     std::vector<double> sy0(std::max(nsrc, 1)), cy0(std::max(nsrc, 1));
     std::vector<double> cdl((size_t)std::max(nsrc, 1) * nx), sdl((size_t)std::max(nsrc, 1) * nx);
     for (int s = 0; s < nsrc; s++) {
@@ -308,6 +358,7 @@ int plan_events(sa_plan* P, int ne, const double* evlo, const double* evla, cons
     SA_CUDA(P->stlo.upload(stlo, nsta, st));
     SA_CUDA(P->stla.upload(stla, nsta, st));
     SA_CUDA(P->cos_stla.upload(cst.data(), nsta, st));
+    TempScope temp(ctx, st);
     DArr<double> d_sy0, d_cy0, d_cdl, d_sdl;
     SA_CUDA(d_sy0.upload(sy0.data(), nsrc, st));
     SA_CUDA(d_cy0.upload(cy0.data(), nsrc, st));
@@ -322,32 +373,39 @@ int plan_events(sa_plan* P, int ne, const double* evlo, const double* evla, cons
         // plan; T, residuals and adjoint fields are then bit-identical.
         SA_CUDA(P->Gx64.alloc(ng));
         SA_CUDA(P->Gy64.alloc(ng));
-        std::vector<double> hG(ng), hGx(ng), hGy(ng), sy(ny), cy(ny);
-        SA_CUDA(cudaMemcpy(sy.data(), P->siny.p, ny * sizeof(double), cudaMemcpyDeviceToHost));
-        SA_CUDA(cudaMemcpy(cy.data(), P->cosy.p, ny * sizeof(double), cudaMemcpyDeviceToHost));
-        const int nth = std::max(1, std::min<int>((int)std::thread::hardware_concurrency(), 64));
+        std::vector<double> hG(ng), hGx(ng), hGy(ng);
+        const std::vector<double>&sy = P->h_siny, &cy = P->h_cosy;
+        // rows of all sources, dealt out to threads of 8192 cells or more (a
+        // cell is about 40 ns, a thread 20 us to start)
+        const size_t rows = (size_t)nsrc * ny;
+        const size_t nth = std::max<size_t>(
+            1, std::min({(size_t)std::thread::hardware_concurrency(), (size_t)64,
+                         rows * nx / 8192}));
+        auto work = [&](size_t t) {
+            for (size_t r = t; r < rows; r += nth) {
+                const size_t s = r / ny;
+                const int iy = (int)(r % ny);
+                for (int ix = 0; ix < nx; ix++) {
+                    const size_t i = s * n + (size_t)iy * nx + ix;
+                    const double cdlv = cdl[s * nx + ix];
+                    const double sdlv = sdl[s * nx + ix];
+                    const double tmp = sy[iy] * sy0[s] + cy[iy] * cy0[s] * cdlv;
+                    const double tmp_c = std::max(-1.0, std::min(1.0, tmp));
+                    hG[i] = std::acos(tmp_c) * R_EARTH;
+                    const double sin_d = std::sqrt(std::max(0.0, 1.0 - tmp_c * tmp_c));
+                    if (sin_d < 1e-14) {
+                        hGx[i] = 0.0;
+                        hGy[i] = 0.0;
+                    } else {
+                        hGx[i] = cy[iy] * cy0[s] * sdlv / sin_d * R_EARTH;
+                        hGy[i] = -(cy[iy] * sy0[s] - sy[iy] * cy0[s] * cdlv) / sin_d * R_EARTH;
+                    }
+                }
+            }
+        };
         std::vector<std::thread> pool;
-        for (int t = 0; t < nth; t++)
-            pool.emplace_back([&, t]() {
-                for (int s = t; s < nsrc; s += nth)
-                    for (int iy = 0; iy < ny; iy++)
-                        for (int ix = 0; ix < nx; ix++) {
-                            const size_t i = (size_t)s * n + (size_t)iy * nx + ix;
-                            const double cdlv = cdl[(size_t)s * nx + ix];
-                            const double sdlv = sdl[(size_t)s * nx + ix];
-                            const double tmp = sy[iy] * sy0[s] + cy[iy] * cy0[s] * cdlv;
-                            const double tmp_c = std::max(-1.0, std::min(1.0, tmp));
-                            hG[i] = std::acos(tmp_c) * R_EARTH;
-                            const double sin_d = std::sqrt(std::max(0.0, 1.0 - tmp_c * tmp_c));
-                            if (sin_d < 1e-14) {
-                                hGx[i] = 0.0;
-                                hGy[i] = 0.0;
-                            } else {
-                                hGx[i] = cy[iy] * cy0[s] * sdlv / sin_d * R_EARTH;
-                                hGy[i] = -(cy[iy] * sy0[s] - sy[iy] * cy0[s] * cdlv) / sin_d * R_EARTH;
-                            }
-                        }
-            });
+        for (size_t t = 1; t < nth; t++) pool.emplace_back(work, t);
+        work(0);
         for (auto& th : pool) th.join();
         if (nsrc) {
             SA_CUDA(cudaMemcpyAsync(P->G64.p, hG.data(), ng * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -387,11 +445,13 @@ int plan_events(sa_plan* P, int ne, const double* evlo, const double* evla, cons
     const int maxs = P->prec == SA_FP64 ? batch64_max_slots(ctx->device) : batch32_max_slots(ctx->device);
     P->slot_bytes = P->prec == SA_FP64 ? batch64_slot_bytes(nx, ny, P->maxr)
                                        : batch32_slot_bytes(nx, ny, P->maxr);
-    size_t fr = 0, tot = 0;
-    SA_CUDA(cudaMemGetInfo(&fr, &tot));
-    const size_t budget = fr / 10 * 7;
     int ns = std::min(maxs, std::max(ne, 1));
-    while (ns > 1 && (size_t)ns * P->slot_bytes > budget) ns--;
+    if (ns > 1) {
+        size_t fr = 0, tot = 0;
+        SA_CUDA(cudaMemGetInfo(&fr, &tot));
+        const size_t budget = fr / 10 * 7;
+        while (ns > 1 && (size_t)ns * P->slot_bytes > budget) ns--;
+    }
     P->nslots = ns;
     SA_CUDA(P->scratch.alloc((size_t)ns * P->slot_bytes));
     // the adjoint-source plane of every slot must start at zero
@@ -1047,6 +1107,8 @@ extern "C" int sa_forward_for_events(sa_ctx* ctx, int precision, int nx, int ny,
                                      const double* weight, int calc_adj, double* syn,
                                      double* adj_s, double* chi, int* fwd_iters,
                                      int* adj_iters) {
+    if (!ctx) return SA_ERR_ARG;
+    TempScope temp(ctx, ctx->stream);   // the plan lives for this call
     sa_plan* P = nullptr;
     int rc = sa_plan_create(ctx, precision, nx, ny, nper, xx_deg, yy_deg, ne, evlo, evla, iper,
                             rec_ptr, rec_idx, nsta, stlo, stla, &P);
@@ -1112,6 +1174,7 @@ int single_solve(sa_ctx* ctx, int precision, int nx, int ny, const double* xx_de
     std::vector<int> rp = {0, nr}, ri(std::max(nr, 1));
     for (int i = 0; i < nr; i++) ri[i] = i;
     const int iper = 0;
+    TempScope temp(ctx, ctx->stream);   // the plan lives for this call
     sa_plan* P = nullptr;
     int rc = sa_plan_create(ctx, precision, nx, ny, 1, xx_deg, yy_deg, 1, &x0, &y0, &iper,
                             rp.data(), ri.data(), nr, nr ? xrec : nullptr, nr ? yrec : nullptr, &P);
@@ -1293,6 +1356,7 @@ extern "C" int sa_depthkernel_columns_group(sa_ctx* ctx, int nx, int ny, int nz,
         t3[2 * nper + i] = periods[i] * (1.0 - 0.5 * dt);
     }
     const size_t plane = (size_t)nx * ny * nper;
+    TempScope temp(ctx, st);
     DArr<double> dper, cps;
     DArr<int> st3;
     SA_CUDA(dper.upload(t3.data(), t3.size(), st));
@@ -1340,6 +1404,7 @@ extern "C" int sa_depthkernel_columns_love(sa_ctx* ctx, int nx, int ny, int nz,
     }
     const int nrun = igr ? 3 : 1;
     const size_t plane = (size_t)nx * ny * nper, ncol = (size_t)nx * ny;
+    TempScope temp(ctx, st);
     DArr<double> dper, cps;
     DArr<int> st3;
     SA_CUDA(dper.upload(t3.data(), t3.size(), st));
@@ -1799,7 +1864,8 @@ extern "C" int sa_pde_smooth(sa_ctx* ctx, int nx, int ny, int nz, double dx_deg,
     const double dz2_inv = 1.0 / (dz_km * dz_km);
     const double dy_inv_half = 1.0 / (2.0 * dy_deg);
     const double dz_inv_half = 1.0 / (2.0 * dz_km);
-    std::vector<double> rowX(ny, 0.0), rowY(ny, 0.0), depE(nz, 0.0);
+    std::vector<double> fac(2 * (size_t)ny + nz, 0.0);
+    double *rowX = fac.data(), *rowY = rowX + ny, *depE = rowY + ny;
     for (int iy = 1; iy < ny - 1; ++iy) {
         const double lat_rad = (ygrid[0] + iy * dy_deg) * DEG2RAD_D;   // src/decomposer.cpp:116-118
         const double cos_lat = std::cos(lat_rad);
@@ -1812,16 +1878,16 @@ extern "C" int sa_pde_smooth(sa_ctx* ctx, int nx, int ny, int nz, double dx_deg,
         const double r_inv = 2.0 / (R_EARTH - zgrid[k]);
         depE[k] = cv * r_inv * dz_inv_half;
     }
-    DArr<double> d_rx, d_ry, d_de, d_work;
-    SA_CUDA(d_rx.upload(rowX.data(), ny, st));
-    SA_CUDA(d_ry.upload(rowY.data(), ny, st));
-    SA_CUDA(d_de.upload(depE.data(), nz, st));
+    TempScope temp(ctx, st);
+    DArr<double> d_fac, d_work;
+    SA_CUDA(d_fac.upload(fac.data(), fac.size(), st));
+    const double *d_rx = d_fac.p, *d_ry = d_rx + ny, *d_de = d_ry + ny;
     double* w = work;
     if (!w) {
         SA_CUDA(d_work.alloc((size_t)nx * ny * nz));
         w = d_work.p;
     }
-    SA_CUDA(launch_pde_smooth(nx, ny, nz, ch * dy2_inv, cv * dz2_inv, d_rx.p, d_ry.p, d_de.p, ns,
+    SA_CUDA(launch_pde_smooth(nx, ny, nz, ch * dy2_inv, cv * dz2_inv, d_rx, d_ry, d_de, ns,
                               field, w, st));
     // the factor arrays (and an internal work array) are released on return
     SA_CUDA(cudaStreamSynchronize(st));
@@ -2082,6 +2148,7 @@ extern "C" int sa_grid_topography(sa_ctx* ctx, int nx_raw, int ny_raw, const dou
         return fail(ctx, SA_ERR_ARG, "Model grid extends beyond topography bounds");
     SA_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
+    TempScope temp(ctx, st);
     DArr<double> dxr, dyr, dzr, dx, dy;
     SA_CUDA(dxr.upload(lon_raw, nx_raw, st));
     SA_CUDA(dyr.upload(lat_raw, ny_raw, st));
@@ -2125,6 +2192,7 @@ extern "C" int sa_topo_media(sa_ctx* ctx, int nx, int ny, const double* lon, con
     for (int ip = 0; even && ip < nper; ip++)
         even = (int)std::min(3.0 * sigma_deg[ip] / h, 1e9) ==
                (int)std::min(3.0 * sigma_deg[ip] / (lon[1] - lon[0]), 1e9);
+    TempScope temp(ctx, st);
     DArr<double> dtab, zs;
     SA_CUDA(dtab.upload(tables.data(), tables.size(), st));
     const double *dlon = dtab.p, *doff = dlon + nx, *dlat = doff + nx, *dsig = dlat + ny;
@@ -2151,6 +2219,7 @@ extern "C" int sa_correct_depth_with_topo(sa_ctx* ctx, int nx, int ny, int nz, i
         return fail(ctx, SA_ERR_ARG, "sa_correct_depth_with_topo: bad sizes (2 <= nz <= 64)");
     SA_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
+    TempScope temp(ctx, st);
     DArr<double> dz;
     SA_CUDA(dz.upload(zgrid, nz, st));
     SA_CUDA(launch_depth_topo(nx, ny, nz, nper, dz.p, angle, sen_vs, sen_vp, sen_rho, st));
