@@ -1547,7 +1547,7 @@ int grad_depth_kernels(sa_grad* g, const double* vs3d, const double* svel, doubl
                         "Love phase-velocity data: the reference's kernels are Rayleigh only "
                         "(src/surf_grid.cpp:282-286, src/surfdisp.cpp:484-487)");
         SA_CUDA(launch_depthkernel(nx, ny, nz, vs3d, nper, g->periods.p, svel, g->lc.p,
-                                   g->sen_vs.p, g->sen_vp.p, g->sen_rho.p, st, sen_hs));
+                                   g->sen_vs.p, g->sen_vp.p, g->sen_rho.p, st, sen_hs, true));
         return SA_OK;
     }
     const size_t plane = (size_t)nx * ny * nper, ncol = (size_t)nx * ny;
@@ -1559,14 +1559,14 @@ int grad_depth_kernels(sa_grad* g, const double* vs3d, const double* svel, doubl
         SA_CUDA(launch_depthkernel_love(nx, ny, nz, vs3d, nper, g->per3.p, g->per3.p + nper,
                                         g->per3.p + 2 * nper, g->cps3.p, g->cps3.p + plane,
                                         g->cps3.p + 2 * plane, 1, g->lc.p, g->sen_vs.p,
-                                        g->sen_rho.p, st));
+                                        g->sen_rho.p, st, true));
         SA_CUDA(cudaMemsetAsync(g->sen_vp.p, 0, plane * nz * sizeof(double), st));
         return SA_OK;
     }
     SA_CUDA(launch_depthkernel_group(nx, ny, nz, vs3d, nper, g->per3.p, g->per3.p + nper,
                                      g->per3.p + 2 * nper, g->cps3.p, g->cps3.p + plane,
                                      g->cps3.p + 2 * plane, g->lc.p, g->sen_vs.p, g->sen_vp.p,
-                                     g->sen_rho.p, st));
+                                     g->sen_rho.p, st, true));
     return SA_OK;
 }
 int grad_ncolst(const sa_grad* g) {

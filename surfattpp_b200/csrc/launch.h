@@ -101,10 +101,11 @@ cudaError_t launch_surfdisp_columns(int nx, int ny, int nz, const double* vs3d, 
                                     const double* periods, int iflsph, int iwave, int igr,
                                     const void* layer_const, double* svel, int* status,
                                     cudaStream_t st);
+// `beside`: another kernel runs at the same time.
 cudaError_t launch_depthkernel(int nx, int ny, int nz, const double* vs3d, int nper,
                                const double* periods, const double* cp, const void* layer_const,
                                double* sen_vs, double* sen_vp, double* sen_rho, cudaStream_t st,
-                               double* sen_hs = nullptr);
+                               double* sen_hs = nullptr, bool beside = false);
 cudaError_t launch_event_cost(int ne, const int* fwd_it, const int* adj_it, unsigned int* key,
                               int* idx, cudaStream_t st);
 // multi-grid queue keys of one level (work = sweeps x cells) and codes
@@ -172,12 +173,12 @@ cudaError_t launch_depthkernel_love(int nx, int ny, int nz, const double* vs3d, 
                                     const double* periods, const double* p1, const double* p2,
                                     const double* cp, const double* cp1, const double* cp2,
                                     int igr, const void* layer_const, double* sen_vs,
-                                    double* sen_rho, cudaStream_t st);
+                                    double* sen_rho, cudaStream_t st, bool beside = false);
 cudaError_t launch_depthkernel_group(int nx, int ny, int nz, const double* vs3d, int nper,
                                      const double* periods, const double* p1, const double* p2,
                                      const double* cp, const double* cp1, const double* cp2,
                                      const void* layer_const, double* sen_vs, double* sen_vp,
-                                     double* sen_rho, cudaStream_t st);
+                                     double* sen_rho, cudaStream_t st, bool beside = false);
 // exact dc/dvs per node from the phase-velocity roots (surfker.cu)
 cudaError_t launch_dispersion_dcdvs(int nx, int ny, int nz, const double* vs3d, int nper,
                                     const double* periods, const double* svel,

@@ -222,10 +222,10 @@ cudaError_t launch_depthkernel_love(int nx, int ny, int nz, const double* vs3d, 
                                     const double* periods, const double* p1, const double* p2,
                                     const double* cp, const double* cp1, const double* cp2,
                                     int igr, const void* layer_const, double* sen_vs,
-                                    double* sen_rho, cudaStream_t st) {
+                                    double* sen_rho, cudaStream_t st, bool beside) {
     const long long n = (long long)nx * ny * nper;
-    depthkernel_love_kernel<<<(unsigned)((n + SK_DEPTH_BLOCK - 1) / SK_DEPTH_BLOCK), SK_DEPTH_BLOCK, 0,
-                              st>>>(
+    const sk::DepthGrid g = sk::depth_grid(n, beside);
+    depthkernel_love_kernel<<<g.blocks, g.threads, 0, st>>>(
         nx, ny, nz, vs3d, nper, periods, p1, p2, cp, cp1, cp2, igr,
         reinterpret_cast<const LayerConst*>(layer_const), sen_vs, sen_rho);
     return cudaGetLastError();
@@ -413,9 +413,10 @@ cudaError_t launch_combine_vs_derivative(int nx, int ny, int nz, int nper, const
 cudaError_t launch_depthkernel(int nx, int ny, int nz, const double* vs3d, int nper,
                                const double* periods, const double* cp, const void* layer_const,
                                double* sen_vs, double* sen_vp, double* sen_rho, cudaStream_t st,
-                               double* sen_hs) {
+                               double* sen_hs, bool beside) {
     const long long n = (long long)nx * ny * nper;
-    depthkernel_kernel<<<(unsigned)((n + SK_DEPTH_BLOCK - 1) / SK_DEPTH_BLOCK), SK_DEPTH_BLOCK, 0, st>>>(
+    const sk::DepthGrid g = sk::depth_grid(n, beside);
+    depthkernel_kernel<<<g.blocks, g.threads, 0, st>>>(
         nx, ny, nz, vs3d, nper, periods, cp, reinterpret_cast<const LayerConst*>(layer_const),
         sen_vs, sen_vp, sen_rho, sen_hs);
     return cudaGetLastError();

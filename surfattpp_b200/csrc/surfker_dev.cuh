@@ -1032,6 +1032,29 @@ __device__ inline void svfunc(RW& W, double omega, double wvno) {
 #define SK_DEPTH_BOUNDS __launch_bounds__(64, 10)
 #define SK_PHASE() ((void)0)
 #endif
+// Blocks and threads for n items: as many waves of one block per SM as full
+// blocks would take, all of one size.  The items a thread has are few and its
+// time is long (a chain of FP64 operations, nearly as long with 4 warps on an
+// SM as with 20), so a short last wave, or full blocks on some of the SMs
+// only, costs as much as a full wave.  Rayleigh phase kernels, ms in full
+// blocks / in equal ones: 16,810 items 1.62 / 1.00, 105,444 (1.11 waves) 4.07
+// / 3.32, 228,010 (2.4) 8.17 / 7.67, 1.36 M (14.3) 41.9 / 41.1; group kernels
+// of the first two 5.52 / 3.21 and 13.2 / 10.9.  `beside` another kernel, less
+// than one wave takes full blocks and leaves the other SMs to it (the gradient
+// of 1681 columns x 10 periods with 250 events 5.57 ms, 5.68 in equal blocks).
+struct DepthGrid {
+    unsigned blocks, threads;
+};
+inline DepthGrid depth_grid(long long n, bool beside) {
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const long long full = (long long)nsm * SK_DEPTH_BLOCK;
+    const long long blocks = std::max<long long>((n + full - 1) / full, 1) * nsm;
+    const long long per =
+        beside && n <= full ? SK_DEPTH_BLOCK : ((n + blocks - 1) / blocks + 31) / 32 * 32;
+    return {(unsigned)((n + per - 1) / per), (unsigned)per};
+}
 __device__ inline void svfunc_phased(RW& W, double omega, double wvno) {
     SK_PHASE();
     up(W, omega, wvno);

@@ -122,10 +122,10 @@ cudaError_t launch_depthkernel_group(int nx, int ny, int nz, const double* vs3d,
                                      const double* periods, const double* p1, const double* p2,
                                      const double* cp, const double* cp1, const double* cp2,
                                      const void* layer_const, double* sen_vs, double* sen_vp,
-                                     double* sen_rho, cudaStream_t st) {
+                                     double* sen_rho, cudaStream_t st, bool beside) {
     const long long n = (long long)nx * ny * nper;
-    depthkernel_group_kernel<<<(unsigned)((n + SK_DEPTH_BLOCK - 1) / SK_DEPTH_BLOCK), SK_DEPTH_BLOCK,
-                               0, st>>>(
+    const sk::DepthGrid g = sk::depth_grid(n, beside);
+    depthkernel_group_kernel<<<g.blocks, g.threads, 0, st>>>(
         nx, ny, nz, vs3d, nper, periods, p1, p2, cp, cp1, cp2,
         reinterpret_cast<const LayerConst*>(layer_const), sen_vs, sen_vp, sen_rho);
     return cudaGetLastError();
