@@ -84,6 +84,10 @@ __device__ __forceinline__ unsigned fdiv_q(unsigned n, const FastDiv& f) {
 // row, column and depth of a cell from two multiply-high divisions instead
 // of 64-bit divisions, which made the index arithmetic the bulk of the
 // instructions.
+// Fields of some 60 000 to 2 million cells are bound by the launch of each
+// step (about 2 us of kernel): launched as a programmatic dependent, a step's
+// blocks are set up while the step before runs.  61x70x30 4.56 -> 3.60 us a
+// step, 100x90x33 4.62 -> 3.28, 31x300x15 4.49 -> 2.47, 301x260x17 8.7 -> 7.2.
 __global__ void __launch_bounds__(256) pde_step_kernel32(PdeConst P, FastDiv fz, FastDiv fy,
                                                          const double* __restrict__ u,
                                                          double* __restrict__ out,
@@ -92,6 +96,8 @@ __global__ void __launch_bounds__(256) pde_step_kernel32(PdeConst P, FastDiv fz,
                                                          const double* __restrict__ depE) {
     const unsigned n = (unsigned)P.nx * P.ny * P.nz;
     const unsigned sy = (unsigned)P.nz, sx = (unsigned)P.ny * P.nz;
+    cudaTriggerProgrammaticLaunchCompletion();   // (the next step's blocks may come and wait)
+    cudaGridDependencySynchronize();             // the step before is complete
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const unsigned col = fdiv_q(i, fz);
         const int k = (int)(i - col * fz.d);
@@ -298,7 +304,8 @@ pde_boundary_kernel(PdeConst P, const double* u, double* out) {
 // its neighbours write what they update; a thread has one depth of one group,
 // a cluster barrier ends a step.  41x41x30: 2.1 us a step, most of it the
 // barrier and the remote stores before it; a launch per step takes 1.9 us of
-// kernel, 1 of gap and 2 to 3 of the host, which it keeps busy all along.
+// kernel, a gap, and 2 to 3 us of the host, which it keeps busy all along
+// (60 steps 293 us with a launch each, 160 now).
 constexpr int kCluster = 16, kClusterThreads = 1024;
 __global__ void __launch_bounds__(kClusterThreads, 1)
 pde_cluster_kernel(PdeConst P, int G, int W, int nstep, double* field,
@@ -385,7 +392,7 @@ namespace {
 // The cluster form where the field fits: two copies of a block's groups and
 // their margins in its shared memory, a thread for each depth of its groups
 // (fields to about 57 000 cells; with two depths a thread 61x70x30 takes
-// 4.1 us a step, a launch each 3.3).
+// 4.1 us a step, a launch each 3.6).
 cudaError_t try_cluster(const PdeConst& P, int nstep, double* field, const double* rowX,
                         const double* rowY, const double* depE, bool* done, cudaStream_t st) {
     constexpr long long kShared = 227 * 1024;
@@ -442,10 +449,23 @@ cudaError_t launch_pde_smooth(int nx, int ny, int nz, double B, double D, const 
     double* a = field;
     double* b = work;
     auto single = [&]() {
-        if (idx32) pde_step_kernel32<<<blocks, 256, 0, st>>>(P, fz, fy, a, b, rowX, rowY, depE);
+        cudaError_t r = cudaSuccess;
+        if (idx32) {
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[0].val.programmaticStreamSerializationAllowed = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(blocks);
+            cfg.blockDim = dim3(256);
+            cfg.stream = st;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            r = cudaLaunchKernelEx(&cfg, pde_step_kernel32, P, fz, fy, (const double*)a, b, rowX,
+                                   rowY, depE);
+        }
         else pde_step_kernel<<<blocks, 256, 0, st>>>(P, a, b, rowX, rowY, depE);
         std::swap(a, b);
-        return cudaGetLastError();
+        return r != cudaSuccess ? r : cudaGetLastError();
     };
     // Depths in equal tiles of at most 60 and their margins, then as many rows
     // as a block's threads hold in equal tiles, then the planes in as many
@@ -463,9 +483,9 @@ cudaError_t launch_pde_smooth(int nx, int ny, int nz, double B, double D, const 
     L.tx = std::max((nx - 2 + ranges - 1) / ranges, 16);
     const long long nr = (nx - 2 + L.tx - 1) / L.tx;
     // Two steps a pass where a pass has planes enough to fill its pipeline and
-    // the blocks their threads: 301x301x40 13 us a step against 17,
-    // 200x180x40 7.8 against 7.6 (and a launch gap), 150x140x30 7.8 against
-    // 4.5, the latency of a range's planes being the same.
+    // the blocks their threads: 301x301x40 13 us a step against 16,
+    // 301x260x17 8.3 against 7.2, 200x180x40 7.8 against 7.7, 150x140x30 7.8
+    // against 4.7, the latency of a range's planes being the same.
     if (n < (1ull << 21) || 2 * L.groups * L.zl < PASS_THREADS || nr * L.tx < 32 || nr > 65535) {
         for (int s = 0; s < nstep; s++)
             if ((e = single()) != cudaSuccess) return e;
