@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <array>
 #include <map>
+#include <mutex>
 #include <cstring>
 #include <string>
 #include <thread>
@@ -39,7 +40,8 @@ int fail(sa_ctx* ctx, int code, const std::string& msg);
 // Where the arrays of one call come from: a TempScope makes the DArrs that its
 // thread constructs while it lives take their memory from the context's pool,
 // in the order of the call's stream.  The pool keeps at most kPoolKeep bytes
-// between calls and ends with the context.  (cudaMalloc and cudaFree take 10
+// between calls (a call that took more gives the rest back before it returns)
+// and ends with the context.  (cudaMalloc and cudaFree take 10
 // to 100 us each and cudaFree waits for the device: a single solve has 52 of
 // each, 41x41 forward and adjoint 6.4 -> 3.4 ms with the pool.)
 constexpr uint64_t kPoolKeep = 256ull << 20;
@@ -52,7 +54,7 @@ struct TempScope {
     TempPool before = t_temp;
     TempScope(sa_ctx* ctx, cudaStream_t st);
     TempScope(const TempScope&) = delete;
-    ~TempScope() { t_temp = before; }
+    ~TempScope();
 };
 
 template <class T>
@@ -112,6 +114,7 @@ struct sa_ctx {
     PeriodCache pc;
     DArr<double> red;   // reduction scratch of the optimizer entry points
     double* red_host = nullptr;   // and their results (pinned)
+    std::mutex red_mutex;         // one of them at a time
     // launch configuration chosen by sa_plan_autotune per grid size:
     // (nx, ny, precision) -> (variant, active slots; 0 = all)
     std::map<std::array<int, 3>, std::array<int, 2>> tune;
@@ -124,6 +127,17 @@ int fail(sa_ctx* ctx, int code, const std::string& msg) {
 }
 
 TempScope::TempScope(sa_ctx* ctx, cudaStream_t st) { t_temp = {ctx->pool, st}; }
+TempScope::~TempScope() {
+    const TempPool own = t_temp;
+    t_temp = before;
+    uint64_t held = 0;
+    if (!own.pool || before.pool ||
+        cudaMemPoolGetAttribute(own.pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        held <= kPoolKeep)
+        return;
+    cudaStreamSynchronize(own.st);   // (memory that is still in use stays)
+    cudaMemPoolTrimTo(own.pool, kPoolKeep);
+}
 
 struct GraphKey {
     const void* ptr[17];
@@ -2035,6 +2049,7 @@ extern "C" int sa_lbfgs_direction(sa_lbfgs* L, int iter, double* dir) {
 extern "C" int sa_dot(sa_ctx* ctx, size_t n, const double* a, const double* b, double* out) {
     if (!ctx || !a || !b || !out) return SA_ERR_ARG;
     SA_CUDA(cudaSetDevice(ctx->device));
+    std::lock_guard<std::mutex> lock(ctx->red_mutex);
     int rc = ctx_red(ctx);
     if (rc) return rc;
     SA_CUDA(launch_dot(n, a, b, ctx->red.p, ctx->red_host, ctx->stream));
@@ -2047,6 +2062,7 @@ extern "C" int sa_kernel_precondition(sa_ctx* ctx, size_t n, const double* ker_d
                                       void* stream) {
     if (!ctx || !ker_den || !ker) return SA_ERR_ARG;
     SA_CUDA(cudaSetDevice(ctx->device));
+    std::lock_guard<std::mutex> lock(ctx->red_mutex);
     int rc = ctx_red(ctx);
     if (rc) return rc;
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
@@ -2057,6 +2073,7 @@ extern "C" int sa_kernel_precondition(sa_ctx* ctx, size_t n, const double* ker_d
 extern "C" int sa_grad_normalization(sa_ctx* ctx, size_t n, double* g, double* max_out) {
     if (!ctx || !g) return SA_ERR_ARG;
     SA_CUDA(cudaSetDevice(ctx->device));
+    std::lock_guard<std::mutex> lock(ctx->red_mutex);
     int rc = ctx_red(ctx);
     if (rc) return rc;
     SA_CUDA(launch_normalise(n, g, ctx->red.p, ctx->red_host, ctx->stream));
@@ -2069,6 +2086,7 @@ extern "C" int sa_descent_angle(sa_ctx* ctx, size_t n, const double* dir, const 
                                 double* deg) {
     if (!ctx || !dir || !grad || !deg) return SA_ERR_ARG;
     SA_CUDA(cudaSetDevice(ctx->device));
+    std::lock_guard<std::mutex> lock(ctx->red_mutex);
     int rc = ctx_red(ctx);
     if (rc) return rc;
     SA_CUDA(launch_dots3(n, grad, dir, ctx->red.p, ctx->red_host, ctx->stream));

@@ -65,7 +65,6 @@ def test_bounded_and_given_back(gpu):
         _smooth(f, ctx)
         _smooth(f[:300].clone(), ctx)
     torch.cuda.empty_cache()
-    torch.cuda.synchronize()
     assert start - torch.cuda.mem_get_info()[0] <= (256 + 32) * MIB
     ctx.close()
     torch.cuda.empty_cache()

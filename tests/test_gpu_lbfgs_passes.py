@@ -60,6 +60,30 @@ def test_direction(gpu, orc, order, n):
     assert np.abs(d - ref).max() <= 1e-11 * np.abs(ref).max()
 
 
+def test_reductions_from_threads(gpu):
+    """One context, many threads: each gets its own sums."""
+    import threading
+    import torch
+    from surfattpp_b200 import optimize
+    x = [torch.full((5000 + i,), float(i + 1), dtype=torch.float64, device="cuda:0")
+         for i in range(6)]
+    one = [torch.ones_like(v) for v in x]
+    torch.cuda.synchronize()
+    bad = []
+
+    def run(i):
+        for _ in range(50):
+            if optimize.dot(x[i], one[i]) != (5000 + i) * (i + 1):
+                bad.append(i)
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+
+
 @pytest.mark.parametrize("n", [1, 255, 257, GRID, GRID + 1])
 def test_reductions(gpu, orc, n):
     from surfattpp_b200 import optimize
