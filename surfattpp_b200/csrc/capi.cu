@@ -1376,9 +1376,8 @@ extern "C" int sa_depthkernel_columns_group(sa_ctx* ctx, int nx, int ny, int nz,
     SA_CUDA(dper.upload(t3.data(), t3.size(), st));
     SA_CUDA(cps.alloc(3 * plane));
     SA_CUDA(st3.alloc(3 * (size_t)nx * ny));
-    for (int k = 0; k < 3; k++)
-        SA_CUDA(launch_surfdisp_columns(nx, ny, nz, vs3d, nper, dper.p + k * nper, 1, 2, 0, L,
-                                        cps.p + k * plane, st3.p + k * (size_t)nx * ny, st));
+    SA_CUDA(launch_surfdisp_columns(nx, ny, nz, vs3d, nper, dper.p, 1, 2, 0, L, cps.p, st3.p, st,
+                                    3));
     SA_CUDA(launch_depthkernel_group(nx, ny, nz, vs3d, nper, dper.p, dper.p + nper,
                                      dper.p + 2 * nper, cps.p, cps.p + plane, cps.p + 2 * plane, L,
                                      sen_vs, sen_vp, sen_rho, st));
@@ -1425,9 +1424,9 @@ extern "C" int sa_depthkernel_columns_love(sa_ctx* ctx, int nx, int ny, int nz,
     SA_CUDA(cps.alloc(3 * plane));
     SA_CUDA(st3.alloc(3 * ncol));
     SA_CUDA(cudaMemsetAsync(st3.p, 0, 3 * ncol * sizeof(int), st));
-    for (int k = 0; k < nrun; k++)   // Love phase velocities (iwave 1)
-        SA_CUDA(launch_surfdisp_columns(nx, ny, nz, vs3d, nper, dper.p + k * nper, 1, 1, 0, L,
-                                        cps.p + k * plane, st3.p + k * ncol, st));
+    // Love phase velocities (iwave 1)
+    SA_CUDA(launch_surfdisp_columns(nx, ny, nz, vs3d, nper, dper.p, 1, 1, 0, L, cps.p, st3.p, st,
+                                    nrun));
     SA_CUDA(launch_depthkernel_love(nx, ny, nz, vs3d, nper, dper.p, dper.p + nper,
                                     dper.p + 2 * nper, cps.p, cps.p + plane, cps.p + 2 * plane,
                                     igr, L, sen_vs, sen_rho, st));
@@ -1565,10 +1564,8 @@ int grad_depth_kernels(sa_grad* g, const double* vs3d, const double* svel, doubl
         return SA_OK;
     }
     const size_t plane = (size_t)nx * ny * nper, ncol = (size_t)nx * ny;
-    for (int k = 0; k < 3; k++)
-        SA_CUDA(launch_surfdisp_columns(nx, ny, nz, vs3d, nper, g->per3.p + k * nper, 1,
-                                        g->iwave, 0, g->lc.p, g->cps3.p + k * plane,
-                                        g->colst.p + (k + 1) * ncol, st));
+    SA_CUDA(launch_surfdisp_columns(nx, ny, nz, vs3d, nper, g->per3.p, 1, g->iwave, 0, g->lc.p,
+                                    g->cps3.p, g->colst.p + ncol, st, 3));
     if (g->iwave == 1) {   // Love group kernels (no vp kernel)
         SA_CUDA(launch_depthkernel_love(nx, ny, nz, vs3d, nper, g->per3.p, g->per3.p + nper,
                                         g->per3.p + 2 * nper, g->cps3.p, g->cps3.p + plane,

@@ -97,10 +97,12 @@ namespace sa {
 // surfker.cu
 size_t layer_const_bytes();
 int build_layer_const(int nz, const double* zgrid, void* out);
+// `runs` period lists of nper, one after another, and as many velocity
+// planes and statuses.
 cudaError_t launch_surfdisp_columns(int nx, int ny, int nz, const double* vs3d, int nper,
                                     const double* periods, int iflsph, int iwave, int igr,
                                     const void* layer_const, double* svel, int* status,
-                                    cudaStream_t st);
+                                    cudaStream_t st, int runs = 1);
 // `beside`: another kernel runs at the same time.
 cudaError_t launch_depthkernel(int nx, int ny, int nz, const double* vs3d, int nper,
                                const double* periods, const double* cp, const void* layer_const,

@@ -49,6 +49,9 @@ surfdisp_columns_kernel(int nx, int ny, int nz, const double* __restrict__ vs3d,
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = col < nx * ny;
     const LayerConst& L = *Lp;
+    periods += (size_t)blockIdx.y * nper;   // blockIdx.y: the run
+    svel += (size_t)blockIdx.y * nx * ny * nper;
+    if (status) status += (size_t)blockIdx.y * nx * ny;
     const size_t pos = live ? (size_t)(col / ny) + (size_t)nx * (col % ny) : 0;
     const int ifunc = iwave == 1 ? 1 : 2;
     sk::SDModel M;
@@ -290,6 +293,9 @@ surfdisp_groups_kernel(int nx, int ny, int nz, const double* __restrict__ vs3d, 
     const unsigned gmask = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
     const int col = blockIdx.x * (kGroupThreads / G) + grp;
     const bool live = col < nx * ny;
+    periods += (size_t)blockIdx.y * nper;   // blockIdx.y: the run
+    svel += (size_t)blockIdx.y * nx * ny * nper;
+    if (status) status += (size_t)blockIdx.y * nx * ny;
     const size_t pos = live ? (size_t)(col / ny) + (size_t)nx * (col % ny) : 0;
     const bool love = iwave == 1;
     double* dp = reinterpret_cast<double*>(reinterpret_cast<char*>(smem4) +
@@ -424,7 +430,7 @@ surfdisp_groups_kernel(int nx, int ny, int nz, const double* __restrict__ vs3d, 
 }
 
 template <int G>
-cudaError_t launch_groups(int nx, int ny, int nz, const double* vs3d, int nper,
+cudaError_t launch_groups(int nx, int ny, int nz, const double* vs3d, int nper, int runs,
                           const double* periods, int iflsph, int iwave, int igr,
                           const LayerConst* Lp, double* svel, int* status, cudaStream_t st) {
     const int per = kGroupThreads / G, n = nx * ny;
@@ -432,7 +438,7 @@ cudaError_t launch_groups(int nx, int ny, int nz, const double* vs3d, int nper,
     cudaError_t e = cudaFuncSetAttribute(surfdisp_groups_kernel<G>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
-    surfdisp_groups_kernel<G><<<(n + per - 1) / per, kGroupThreads, bytes, st>>>(
+    surfdisp_groups_kernel<G><<<dim3((n + per - 1) / per, runs), kGroupThreads, bytes, st>>>(
         nx, ny, nz, vs3d, nper, periods, iflsph, iwave, igr, Lp, svel, status);
     return cudaGetLastError();
 }
@@ -442,8 +448,9 @@ cudaError_t launch_groups(int nx, int ny, int nz, const double* vs3d, int nper,
 cudaError_t launch_surfdisp_columns(int nx, int ny, int nz, const double* vs3d, int nper,
                                     const double* periods, int iflsph, int iwave, int igr,
                                     const void* layer_const, double* svel, int* status,
-                                    cudaStream_t st) {
+                                    cudaStream_t st, int runs) {
     const int n = nx * ny;
+    const long long all = (long long)n * runs;
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -458,14 +465,20 @@ cudaError_t launch_surfdisp_columns(int nx, int ny, int nz, const double* vs3d, 
     // lanes: 1681 columns x 10 periods 2.37 / 2.50 / 3.15 / 15.8; 3233 x 8
     // 3.80 / 2.30 / 2.69 / 12.4; 8787 x 12 14.6 / 9.3 / 6.6 / 19.0; 20,687 x
     // 12 36 / 23 / 17.8 / 26.1; 40,401 x 15 85 / 52 / 36.7 / 34.8.
-    auto groups = n <= 16 * nsm    ? launch_groups<32>
-                  : n <= 32 * nsm  ? launch_groups<16>
-                  : n <= 240 * nsm ? launch_groups<8>
-                                   : nullptr;
+    // Several runs (the three period lists of the group kernels) count as
+    // that many columns: in one launch they fill the SMs that one run leaves
+    // idle (group kernels with their runs, Rayleigh / Love: 41x41x30 with 10
+    // periods 10.0 -> 7.5 / 5.2 -> 3.1 ms, 101x87x33 with 12 31.1 -> 30.4 /
+    // 12.3 -> 11.9, 151x151x30 with 8 50.5 -> 38.5 / 20.5 -> 12.9).
+    auto groups = all <= 16 * nsm    ? launch_groups<32>
+                  : all <= 32 * nsm  ? launch_groups<16>
+                  : all <= 240 * nsm ? launch_groups<8>
+                                     : nullptr;
     if (groups)
-        return groups(nx, ny, nz, vs3d, nper, periods, iflsph, iwave, igr, Lp, svel, status, st);
-    surfdisp_columns_kernel<<<(n + 63) / 64, 64, 0, st>>>(nx, ny, nz, vs3d, nper, periods, iflsph,
-                                                          iwave, igr, Lp, svel, status);
+        return groups(nx, ny, nz, vs3d, nper, runs, periods, iflsph, iwave, igr, Lp, svel, status,
+                      st);
+    surfdisp_columns_kernel<<<dim3((n + 63) / 64, runs), 64, 0, st>>>(
+        nx, ny, nz, vs3d, nper, periods, iflsph, iwave, igr, Lp, svel, status);
     return cudaGetLastError();
 }
 

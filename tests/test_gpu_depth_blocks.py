@@ -1,6 +1,8 @@
 """GPU: the depth kernels in blocks of equal size, whatever the number of
 (column, period) items: a single item, counts around a warp, around one full
-wave (148 blocks of 640 threads) and beyond it.
+wave (148 blocks of 640 threads) and beyond it; the group kernels' three
+phase-velocity runs in one launch of each form (32, 16, 8 lanes and a thread
+per column).
 
 The columns repeat a few columns in an order that puts each beside others, and
 every copy's kernels must be those of the column's first copy in the smallest
@@ -22,6 +24,7 @@ def _columns():
 
 @pytest.mark.parametrize("kind", ["phase", "group", "love"])
 @pytest.mark.parametrize("nx,ny,nper", [(1, 1, 1), (1, 31, 1), (3, 11, 1), (149, 1, 2),
+                                        (33, 31, 2), (60, 61, 2),
                                         (320, 148, 2), (320, 74, 4), (57, 1662, 1),
                                         (500, 97, 2), (480, 148, 4)])
 def test_equal_blocks(gpu, orc, kind, nx, ny, nper):
