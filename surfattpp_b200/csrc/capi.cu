@@ -2202,8 +2202,9 @@ extern "C" int sa_topo_media(sa_ctx* ctx, int nx, int ny, const double* lon, con
     }
     tables.insert(tables.end(), lat, lat + ny);
     tables.insert(tables.end(), sigma_deg, sigma_deg + nper);
-    // (the window's width in points must be the one lon[1] - lon[0] gives)
-    bool even = h > 0.0 && worst <= 1e-9 * smin && gauss_rows_fits(nx, nper);
+    // (the window's width in points must be an int, the one lon[1] - lon[0] gives)
+    bool even = h > 0.0 && worst <= 1e-9 * smin && 3.0 * smax / h < 1e9 &&
+                gauss_rows_fits(nx, nper);
     for (int ip = 0; even && ip < nper; ip++)
         even = (int)std::min(3.0 * sigma_deg[ip] / h, 1e9) ==
                (int)std::min(3.0 * sigma_deg[ip] / (lon[1] - lon[0]), 1e9);

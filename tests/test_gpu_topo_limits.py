@@ -1,0 +1,38 @@
+"""sa_topo_media at the ends of what it accepts: windows wider than any
+grid.  Bars: media within 1e-12 and dip angles within 1e-9 degrees of the
+oracle, the bars of the ordinary cases; non-finite values in the same cells as
+the oracle's."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _media(x, y, z, sig):
+    import torch
+    from surfattpp_b200 import surfgrid
+    zt = torch.as_tensor(z, device="cuda:0")
+    return [v.cpu().numpy() for v in surfgrid.build_media_with_topo(x, y, zt, np.asarray(sig))]
+
+
+def _match(got, ref):
+    for a, b, tol in zip(got, ref, (1e-12, 1e-12, 1e-12, 1e-9)):
+        f = np.isfinite(b)
+        assert np.array_equal(np.isfinite(a), f)
+        assert np.array_equal(np.isnan(a), np.isnan(b))
+        assert np.abs(a[f] - b[f]).max() <= tol
+
+
+def _grid(nx, ny, seed):
+    g = np.random.default_rng(seed)
+    return 102.0 + 0.01 * np.arange(nx), 24.0 + 0.013 * np.arange(ny), g.uniform(0, 4, (ny, nx))
+
+
+@pytest.mark.parametrize("wide", [1e8, 1e30, np.inf])
+def test_window_beyond_integers(gpu, orc, wide):
+    """Beside a period whose window in grid points exceeds an integer, the
+    others come out as ever."""
+    x, y, z = _grid(70, 33, 1)
+    got = _media(x, y, z, [0.0123, wide, 0.061])
+    ref = orc.topo_media(x, y, z, np.array([0.0123, 0.061]))
+    _match([a[::2] for a in got], ref)
