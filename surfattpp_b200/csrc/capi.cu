@@ -2189,8 +2189,9 @@ extern "C" int sa_topo_media(sa_ctx* ctx, int nx, int ny, const double* lon, con
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     const size_t n = (size_t)nx * ny;
     // An evenly spaced longitude grid (up to rounding: 1e-9 of the smallest
-    // sigma) shares a row's weights between its cells; others weigh every
-    // point of every cell.
+    // sigma) shares a row's weights between its cells; others, and grids with
+    // a coordinate that is not finite (a point without weight, which must not
+    // enter the shared sums), weigh every point of every cell.
     const double h = (lon[nx - 1] - lon[0]) / (nx - 1);
     const double smin = *std::min_element(sigma_deg, sigma_deg + nper);
     const double smax = *std::max_element(sigma_deg, sigma_deg + nper);
@@ -2204,7 +2205,8 @@ extern "C" int sa_topo_media(sa_ctx* ctx, int nx, int ny, const double* lon, con
     tables.insert(tables.end(), sigma_deg, sigma_deg + nper);
     // (the window's width in points must be an int, the one lon[1] - lon[0] gives)
     bool even = h > 0.0 && worst <= 1e-9 * smin && 3.0 * smax / h < 1e9 &&
-                gauss_rows_fits(nx, nper);
+                gauss_rows_fits(nx, nper) &&
+                std::all_of(tables.begin(), tables.end(), [](double v) { return std::isfinite(v); });
     for (int ip = 0; even && ip < nper; ip++)
         even = (int)std::min(3.0 * sigma_deg[ip] / h, 1e9) ==
                (int)std::min(3.0 * sigma_deg[ip] / (lon[1] - lon[0]), 1e9);

@@ -1,7 +1,7 @@
-"""sa_topo_media at the ends of what it accepts: windows wider than any
-grid.  Bars: media within 1e-12 and dip angles within 1e-9 degrees of the
-oracle, the bars of the ordinary cases; non-finite values in the same cells as
-the oracle's."""
+"""sa_topo_media at the ends of what it accepts: windows wider than any grid,
+coordinates that are not finite.  Bars: media within 1e-12 and dip angles
+within 1e-9 degrees of the oracle, the bars of the ordinary cases; non-finite
+values in the same cells as the oracle's."""
 import numpy as np
 import pytest
 
@@ -36,3 +36,15 @@ def test_window_beyond_integers(gpu, orc, wide):
     got = _media(x, y, z, [0.0123, wide, 0.061])
     ref = orc.topo_media(x, y, z, np.array([0.0123, 0.061]))
     _match([a[::2] for a in got], ref)
+
+
+@pytest.mark.parametrize("axis,bad", [("x", np.nan), ("x", np.inf), ("y", np.nan)])
+def test_coordinate_not_finite(gpu, axis, bad):
+    """A point at no position has no weight: cells away from it (and from the
+    gradients that difference it) stay finite."""
+    x, y, z = _grid(70, 33, 2)
+    k = 20
+    (x if axis == "x" else y)[k] = bad
+    for a in _media(x, y, z, [0.061]):
+        keep = np.delete(a, [k - 1, k, k + 1], axis=2 if axis == "x" else 1)
+        assert np.isfinite(keep).all()
