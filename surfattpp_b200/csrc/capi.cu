@@ -2195,7 +2195,7 @@ extern "C" int sa_topo_media(sa_ctx* ctx, int nx, int ny, const double* lon, con
     const double h = (lon[nx - 1] - lon[0]) / (nx - 1);
     const double smin = *std::min_element(sigma_deg, sigma_deg + nper);
     const double smax = *std::max_element(sigma_deg, sigma_deg + nper);
-    std::vector<double> tables(lon, lon + nx);   // lon, off, lat, sigma
+    std::vector<double> tables(lon, lon + nx);   // lon, off, lat, sigma, a zero
     double worst = 0.0;
     for (int m = 0; m < nx; m++) {
         tables.push_back(std::fma(-(double)m, h, lon[m] - lon[0]));
@@ -2210,21 +2210,30 @@ extern "C" int sa_topo_media(sa_ctx* ctx, int nx, int ny, const double* lon, con
     for (int ip = 0; even && ip < nper; ip++)
         even = (int)std::min(3.0 * sigma_deg[ip] / h, 1e9) ==
                (int)std::min(3.0 * sigma_deg[ip] / (lon[1] - lon[0]), 1e9);
+    tables.push_back(0.0);
     TempScope temp(ctx, st);
     DArr<double> dtab, zs;
     SA_CUDA(dtab.upload(tables.data(), tables.size(), st));
     const double *dlon = dtab.p, *doff = dlon + nx, *dlat = doff + nx, *dsig = dlat + ny;
+    int* odd = reinterpret_cast<int*>(dtab.p + tables.size() - 1);
     // each period starts from the unsmoothed gridded topography (:93-96, :113-114)
     SA_CUDA(zs.alloc(n * nper));
+    int h_odd = 0;
     if (even) {
         SA_CUDA(launch_gauss_rows(nx, ny, nper, z_gridded, dlat, doff, h, dsig, smax, zs.p, st));
-    } else {
+        SA_CUDA(launch_topo_media(nx, ny, nper, zs.p, dlon, dlat, m11, m12, m22, angle, odd, st));
+        SA_CUDA(cudaMemcpyAsync(&h_odd, odd, sizeof(int), cudaMemcpyDeviceToHost, st));
+        SA_CUDA(cudaStreamSynchronize(st));
+    }
+    // (the shared weights are zero beyond a window, which a topography that is
+    // not finite does not bear: such a grid is done again point by point)
+    if (!even || h_odd) {
         for (int ip = 0; ip < nper; ip++)
             SA_CUDA(launch_gauss_geo(nx, ny, z_gridded, dlon, dlat, sigma_deg[ip], zs.p + ip * n,
                                      st));
+        SA_CUDA(launch_topo_media(nx, ny, nper, zs.p, dlon, dlat, m11, m12, m22, angle, odd, st));
+        SA_CUDA(cudaStreamSynchronize(st));
     }
-    SA_CUDA(launch_topo_media(nx, ny, nper, zs.p, dlon, dlat, m11, m12, m22, angle, st));
-    SA_CUDA(cudaStreamSynchronize(st));
     return SA_OK;
 }
 

@@ -157,9 +157,10 @@ bool gauss_rows_fits(int nx, int nper);
 cudaError_t launch_gauss_rows(int nx, int ny, int nper, const double* data, const double* lats,
                               const double* off, double h, const double* sigmas, double sigma_max,
                               double* out, cudaStream_t st);
+// *odd is set if a smoothed cell is not finite
 cudaError_t launch_topo_media(int nx, int ny, int nper, const double* z, const double* lon,
                               const double* lat, double* m11, double* m12, double* m22,
-                              double* angle, cudaStream_t st);
+                              double* angle, int* odd, cudaStream_t st);
 cudaError_t launch_depth_topo(int nx, int ny, int nz, int nper, const double* zg,
                               const double* angle, double* k0, double* k1, double* k2,
                               cudaStream_t st);

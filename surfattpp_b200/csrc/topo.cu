@@ -236,14 +236,16 @@ __global__ void gauss_geo_kernel(int nx, int ny, const double* __restrict__ data
     out[i + (size_t)nx * j] = swd / sw;
 }
 
-// block row y: the period
+// block row y: the period.  *odd is set where the smoothed topography is not
+// finite.
 __global__ void media_kernel(int nx, int ny, const double* __restrict__ zs,
                              const double* __restrict__ lon, const double* __restrict__ lat,
-                             double* m11, double* m12, double* m22, double* angle) {
+                             double* m11, double* m12, double* m22, double* angle, int* odd) {
     const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (k >= (size_t)nx * ny) return;
     const size_t plane = blockIdx.y * (size_t)nx * ny;
     const double* z = zs + plane;
+    if (!isfinite(z[k])) *odd = 1;
     m11 += plane;
     m12 += plane;
     m22 += plane;
@@ -357,10 +359,10 @@ bool gauss_rows_fits(int nx, int nper) { return nx <= 2000 && nper <= 65535; }
 
 cudaError_t launch_topo_media(int nx, int ny, int nper, const double* z, const double* lon,
                               const double* lat, double* m11, double* m12, double* m22,
-                              double* angle, cudaStream_t st) {
+                              double* angle, int* odd, cudaStream_t st) {
     const size_t n = (size_t)nx * ny;
     media_kernel<<<dim3((unsigned)((n + 255) / 256), nper), 256, 0, st>>>(nx, ny, z, lon, lat, m11,
-                                                                          m12, m22, angle);
+                                                                          m12, m22, angle, odd);
     return cudaGetLastError();
 }
 

@@ -1,7 +1,7 @@
 """sa_topo_media at the ends of what it accepts: windows wider than any grid,
-coordinates that are not finite.  Bars: media within 1e-12 and dip angles
-within 1e-9 degrees of the oracle, the bars of the ordinary cases; non-finite
-values in the same cells as the oracle's."""
+coordinates and topography that are not finite.  Bars: media within 1e-12 and
+dip angles within 1e-9 degrees of the oracle, the bars of the ordinary cases;
+non-finite values in the same cells as the oracle's."""
 import numpy as np
 import pytest
 
@@ -48,3 +48,15 @@ def test_coordinate_not_finite(gpu, axis, bad):
     for a in _media(x, y, z, [0.061]):
         keep = np.delete(a, [k - 1, k, k + 1], axis=2 if axis == "x" else 1)
         assert np.isfinite(keep).all()
+
+
+@pytest.mark.parametrize("bad", [[np.nan], [np.inf], [-np.inf], [np.inf, -np.inf]])
+@pytest.mark.parametrize("nx,ny", [(31, 12), (70, 33), (263, 9)])
+def test_topography_not_finite(gpu, orc, nx, ny, bad):
+    """A non-finite cell reaches the cells whose window holds it, no others."""
+    x, y, z = _grid(nx, ny, 3)
+    for i, v in enumerate(bad):
+        z[ny // 2, nx // 2 + 3 * i] = v
+    z[0, nx - 1] = bad[0]
+    sig = np.array([0.002, 0.0123, 0.031])
+    _match(_media(x, y, z, sig), orc.topo_media(x, y, z, sig))
