@@ -2205,7 +2205,7 @@ extern "C" int sa_topo_media(sa_ctx* ctx, int nx, int ny, const double* lon, con
     tables.insert(tables.end(), sigma_deg, sigma_deg + nper);
     // (the window's width in points must be an int, the one lon[1] - lon[0] gives)
     bool even = h > 0.0 && worst <= 1e-9 * smin && 3.0 * smax / h < 1e9 &&
-                gauss_rows_fits(nx, nper) &&
+                gauss_rows_fits(nx) &&
                 std::all_of(tables.begin(), tables.end(), [](double v) { return std::isfinite(v); });
     for (int ip = 0; even && ip < nper; ip++)
         even = (int)std::min(3.0 * sigma_deg[ip] / h, 1e9) ==
@@ -2216,22 +2216,37 @@ extern "C" int sa_topo_media(sa_ctx* ctx, int nx, int ny, const double* lon, con
     SA_CUDA(dtab.upload(tables.data(), tables.size(), st));
     const double *dlon = dtab.p, *doff = dlon + nx, *dlat = doff + nx, *dsig = dlat + ny;
     int* odd = reinterpret_cast<int*>(dtab.p + tables.size() - 1);
-    // each period starts from the unsmoothed gridded topography (:93-96, :113-114)
-    SA_CUDA(zs.alloc(n * nper));
+    // each period starts from the unsmoothed gridded topography (:93-96,
+    // :113-114); as many periods at a time as a launch's grid and kPoolKeep
+    // bytes of smoothed planes hold
+    const int some = (int)std::min<size_t>({(size_t)nper, (size_t)65535,
+                                            std::max<size_t>(kPoolKeep / (n * sizeof(double)), 1)});
+    SA_CUDA(zs.alloc(n * some));
+    auto media = [&](bool rows) -> int {
+        for (int ip = 0; ip < nper; ip += some) {
+            const int np = std::min(some, nper - ip);
+            const size_t at = ip * n;
+            if (rows)
+                SA_CUDA(launch_gauss_rows(nx, ny, np, z_gridded, dlat, doff, h, dsig + ip, smax,
+                                          zs.p, st));
+            for (int k = 0; k < np && !rows; k++)
+                SA_CUDA(launch_gauss_geo(nx, ny, z_gridded, dlon, dlat, sigma_deg[ip + k],
+                                         zs.p + k * n, st));
+            SA_CUDA(launch_topo_media(nx, ny, np, zs.p, dlon, dlat, m11 + at, m12 + at, m22 + at,
+                                      angle + at, odd, st));
+        }
+        return SA_OK;
+    };
     int h_odd = 0;
     if (even) {
-        SA_CUDA(launch_gauss_rows(nx, ny, nper, z_gridded, dlat, doff, h, dsig, smax, zs.p, st));
-        SA_CUDA(launch_topo_media(nx, ny, nper, zs.p, dlon, dlat, m11, m12, m22, angle, odd, st));
+        if (const int rc = media(true)) return rc;
         SA_CUDA(cudaMemcpyAsync(&h_odd, odd, sizeof(int), cudaMemcpyDeviceToHost, st));
         SA_CUDA(cudaStreamSynchronize(st));
     }
     // (the shared weights are zero beyond a window, which a topography that is
     // not finite does not bear: such a grid is done again point by point)
     if (!even || h_odd) {
-        for (int ip = 0; ip < nper; ip++)
-            SA_CUDA(launch_gauss_geo(nx, ny, z_gridded, dlon, dlat, sigma_deg[ip], zs.p + ip * n,
-                                     st));
-        SA_CUDA(launch_topo_media(nx, ny, nper, zs.p, dlon, dlat, m11, m12, m22, angle, odd, st));
+        if (const int rc = media(false)) return rc;
         SA_CUDA(cudaStreamSynchronize(st));
     }
     return SA_OK;

@@ -151,9 +151,9 @@ cudaError_t launch_model_update_vs(size_t n, const double* vs, const double* dir
 // topo.cu
 cudaError_t launch_gauss_geo(int nx, int ny, const double* data, const double* lons,
                              const double* lats, double sigma, double* out, cudaStream_t st);
-// all periods' smoothing on an evenly spaced longitude grid (step h, off =
+// nper (at most 65535) periods' smoothing on an evenly spaced longitude grid (step h, off =
 // lon - lon[0] - m h) of a width that gauss_rows_fits
-bool gauss_rows_fits(int nx, int nper);
+bool gauss_rows_fits(int nx);
 cudaError_t launch_gauss_rows(int nx, int ny, int nper, const double* data, const double* lats,
                               const double* off, double h, const double* sigmas, double sigma_max,
                               double* out, cudaStream_t st);

@@ -355,7 +355,7 @@ cudaError_t launch_gauss_rows(int nx, int ny, int nper, const double* data, cons
     return cudaGetLastError();
 }
 
-bool gauss_rows_fits(int nx, int nper) { return nx <= 2000 && nper <= 65535; }
+bool gauss_rows_fits(int nx) { return nx <= 2000; }
 
 cudaError_t launch_topo_media(int nx, int ny, int nper, const double* z, const double* lon,
                               const double* lat, double* m11, double* m12, double* m22,

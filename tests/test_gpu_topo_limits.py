@@ -1,7 +1,8 @@
 """sa_topo_media at the ends of what it accepts: windows wider than any grid,
-coordinates and topography that are not finite.  Bars: media within 1e-12 and
-dip angles within 1e-9 degrees of the oracle, the bars of the ordinary cases;
-non-finite values in the same cells as the oracle's."""
+coordinates and topography that are not finite, more periods than a launch's
+grid holds.  Bars: media within 1e-12 and dip angles within 1e-9 degrees of
+the oracle, the bars of the ordinary cases; non-finite values in the same
+cells as the oracle's."""
 import numpy as np
 import pytest
 
@@ -60,3 +61,13 @@ def test_topography_not_finite(gpu, orc, nx, ny, bad):
     z[0, nx - 1] = bad[0]
     sig = np.array([0.002, 0.0123, 0.031])
     _match(_media(x, y, z, sig), orc.topo_media(x, y, z, sig))
+
+
+def test_more_periods_than_a_grid_holds(gpu, orc):
+    x, y, z = _grid(3, 3, 4)
+    sig = np.full(65540, 0.0123)
+    sig[-1] = 0.031
+    got = _media(x, y, z, sig)
+    _match([a[-2:] for a in got], orc.topo_media(x, y, z, sig[-2:]))
+    for a in got:
+        assert np.array_equal(a[0], a[65535])
