@@ -88,9 +88,10 @@ __device__ __forceinline__ unsigned fdiv_q(unsigned n, const FastDiv& f) {
 // step (about 2 us of kernel): launched as a programmatic dependent, a step's
 // blocks are set up while the step before runs.  61x70x30 4.56 -> 3.60 us a
 // step, 100x90x33 4.62 -> 3.28, 31x300x15 4.49 -> 2.47, 301x260x17 8.7 -> 7.2.
+// (Blocks come while the step before writes u, so u and out are plain
+// pointers: `__restrict__` would let u be read as if it never changed.)
 __global__ void __launch_bounds__(256) pde_step_kernel32(PdeConst P, FastDiv fz, FastDiv fy,
-                                                         const double* __restrict__ u,
-                                                         double* __restrict__ out,
+                                                         const double* u, double* out,
                                                          const double* __restrict__ rowX,
                                                          const double* __restrict__ rowY,
                                                          const double* __restrict__ depE) {
