@@ -52,7 +52,8 @@ struct TempPool {
 thread_local TempPool t_temp;
 struct TempScope {
     TempPool before = t_temp;
-    TempScope(sa_ctx* ctx, cudaStream_t st);
+    const bool trim;   // false: the call takes too little to give any back
+    TempScope(sa_ctx* ctx, cudaStream_t st, bool trim = true);
     TempScope(const TempScope&) = delete;
     ~TempScope();
 };
@@ -126,12 +127,23 @@ int fail(sa_ctx* ctx, int code, const std::string& msg) {
     return code;
 }
 
-TempScope::TempScope(sa_ctx* ctx, cudaStream_t st) { t_temp = {ctx->pool, st}; }
+// While it lives, its thread may allocate although a stream is being captured
+// (its own: the memory is the graph's; another: nothing of it is recorded).
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+TempScope::TempScope(sa_ctx* ctx, cudaStream_t st, bool trim) : trim(trim) {
+    t_temp = {ctx->pool, st};
+}
 TempScope::~TempScope() {
     const TempPool own = t_temp;
     t_temp = before;
     uint64_t held = 0;
-    if (!own.pool || before.pool ||
+    if (!own.pool || before.pool || !trim ||
         cudaMemPoolGetAttribute(own.pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
         held <= kPoolKeep)
         return;
@@ -1911,7 +1923,8 @@ namespace {
 constexpr int LBFGS_STORE = 5;   // MAX_LBFGS_STORE, include/config.h:90
 
 // Reduction scratch and the host words (pinned, device-visible) that the
-// reductions of the optimizer entry points leave their results in.
+// reductions of the optimizer entry points leave their results in; red_mutex
+// is held until a reduction has run.
 int ctx_red(sa_ctx* ctx) {
     if (!ctx->red.p) {
         const size_t n = reduce_scratch_doubles();
@@ -2059,11 +2072,21 @@ extern "C" int sa_kernel_precondition(sa_ctx* ctx, size_t n, const double* ker_d
                                       void* stream) {
     if (!ctx || !ker_den || !ker) return SA_ERR_ARG;
     SA_CUDA(cudaSetDevice(ctx->device));
-    std::lock_guard<std::mutex> lock(ctx->red_mutex);
-    int rc = ctx_red(ctx);
-    if (rc) return rc;
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-    SA_CUDA(launch_kernel_precondition(n, ker_den, ctx->red.p, ker, st));
+    if (!ctx->pool) {
+        std::lock_guard<std::mutex> lock(ctx->red_mutex);
+        if (const int rc = ctx_red(ctx)) return rc;
+        SA_CUDA(launch_kernel_precondition(n, ker_den, ctx->red.p, ker, st));
+        SA_CUDA(cudaStreamSynchronize(st));
+        return SA_OK;
+    }
+    // (returns before its kernels have run: partials of its own, in the order
+    // of its stream, since another call on another stream may run beside it)
+    RelaxedCapture relaxed;
+    TempScope temp(ctx, st, false);
+    DArr<double> partial;
+    SA_CUDA(partial.alloc(red_blocks()));
+    SA_CUDA(launch_kernel_precondition(n, ker_den, partial.p, ker, st));
     return SA_OK;
 }
 

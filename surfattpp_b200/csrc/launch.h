@@ -129,8 +129,10 @@ cudaError_t launch_dots3(size_t n, const double* a, const double* b, double* scr
                          cudaStream_t st);
 // out = max|g|, then g /= max|g| unless that is below DBL_EPSILON
 cudaError_t launch_normalise(size_t n, double* g, double* scratch, double* out, cudaStream_t st);
-// postproc::kernel_precondition of ker by ker_den (scratch: reduction scratch)
-cudaError_t launch_kernel_precondition(size_t n, const double* ker_den, double* scratch,
+// postproc::kernel_precondition of ker by ker_den (partial: red_blocks()
+// doubles that no other call uses until this one has run)
+size_t red_blocks();
+cudaError_t launch_kernel_precondition(size_t n, const double* ker_den, double* partial,
                                        double* ker, cudaStream_t st);
 // The L-BFGS recursion's scalars by pair slot: s.y, y.y, alpha, alpha - beta.
 // A pair has its first iterate's slot, so that it is valid while both are stored.

@@ -238,20 +238,20 @@ unsigned red_grid(size_t n) {
 }
 }  // namespace
 
-cudaError_t launch_kernel_precondition(size_t n, const double* ker_den, double* scratch,
+// partial: red_blocks() doubles of the call's own
+cudaError_t launch_kernel_precondition(size_t n, const double* ker_den, double* partial,
                                        double* ker, cudaStream_t st) {
-    double* partial = scratch + 3 * RED_BLOCKS;
     absmax_kernel<<<red_grid(n), RED_THREADS, 0, st>>>(n, ker_den, partial);
     precondition_kernel<<<red_grid(n), RED_THREADS, 0, st>>>(n, ker_den, partial, ker);
     return cudaGetLastError();
 }
 
-// scratch: the partials of 3 sums, those of the precondition (which may run on
-// a stream of its own), the counter
-size_t reduce_scratch_doubles() { return 4 * RED_BLOCKS + 1; }
+// scratch: the partials of 3 sums, the counter
+size_t red_blocks() { return RED_BLOCKS; }
+size_t reduce_scratch_doubles() { return 3 * RED_BLOCKS + 1; }
 namespace {
 unsigned* red_count(double* scratch) {
-    return reinterpret_cast<unsigned*>(scratch + 4 * RED_BLOCKS);
+    return reinterpret_cast<unsigned*>(scratch + 3 * RED_BLOCKS);
 }
 }  // namespace
 
