@@ -146,6 +146,10 @@ __device__ __forceinline__ void pde_store(const PdeConst& P, double* __restrict_
 constexpr int kRows = 4;
 constexpr int kRing = 5;
 constexpr int PASS_THREADS = 512;   // 128 registers
+constexpr int kPassDepths = 64;     // depths of a block at most
+// bytes of a block at most: kRows rows for each of its threads, two more of
+// kPassDepths and a cell at either end, kRing planes before and 2 after a step
+constexpr int kPassShared = (kRing + 2) * (kRows * PASS_THREADS + 2 * kPassDepths + 2) * 8;
 struct PassTiles {
     int tx, ty, tz;   // interior cells per tile
     int nty;          // tiles along y
@@ -309,6 +313,7 @@ pde_boundary_kernel(PdeConst P, const double* u, double* out) {
 // kernel, a gap, and 2 to 3 us of the host, which it keeps busy all along
 // (60 steps 293 us with a launch each, 160 now).
 constexpr int kCluster = 16, kClusterThreads = 1024;
+constexpr int kClusterShared = 227 * 1024;   // bytes of a block at most
 __global__ void __launch_bounds__(kClusterThreads, 1)
 pde_cluster_kernel(PdeConst P, int G, int W, int nstep, double* field,
                    const double* __restrict__ rowX, const double* __restrict__ rowY,
@@ -391,22 +396,25 @@ pde_cluster_kernel(PdeConst P, int G, int W, int nstep, double* field,
 
 namespace {
 
+// (The limit on a kernel's dynamic shared memory belongs to the device, not to
+// the launch after it, and threads launch at the same time: every call sets
+// the largest that any call needs.)
+
 // The cluster form where the field fits: two copies of a block's groups and
 // their margins in its shared memory, a thread for each depth of its groups
 // (fields to about 57 000 cells; with two depths a thread 61x70x30 takes
 // 4.1 us a step, a launch each 3.6).
 cudaError_t try_cluster(const PdeConst& P, int nstep, double* field, const double* rowX,
                         const double* rowY, const double* depE, bool* done, cudaStream_t st) {
-    constexpr long long kShared = 227 * 1024;
     const long long G = (P.ny + kRows - 1) / kRows, U = (long long)(P.nx - 2) * G;
     const long long W = std::max((U + kCluster - 1) / kCluster, G);
     const long long smem =
         2 * ((W + 2 * G) * kRows * P.nz + kRows * G) * (long long)sizeof(double);
     *done = false;
-    if (smem > kShared || W * (P.nz - 2) > kClusterThreads) return cudaSuccess;
+    if (smem > kClusterShared || W * (P.nz - 2) > kClusterThreads) return cudaSuccess;
     cudaError_t e;
     if ((e = cudaFuncSetAttribute(pde_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem)))
+                                  kClusterShared)))
         return e;
     if ((e = cudaFuncSetAttribute(pde_cluster_kernel,
                                   cudaFuncAttributeNonPortableClusterSizeAllowed, 1)))
@@ -473,7 +481,7 @@ cudaError_t launch_pde_smooth(int nx, int ny, int nz, double B, double D, const 
     // as a block's threads hold in equal tiles, then the planes in as many
     // ranges as there are blocks left.
     PassTiles L;
-    const int ntz = nz <= 64 ? 1 : (nz - 2 + 59) / 60;
+    const int ntz = nz <= kPassDepths ? 1 : (nz - 2 + kPassDepths - 5) / (kPassDepths - 4);
     L.tz = (nz - 2 + ntz - 1) / ntz;
     L.zl = ntz == 1 ? nz : L.tz + 4;
     const int rows = PASS_THREADS / L.zl * kRows - 4;
@@ -498,7 +506,7 @@ cudaError_t launch_pde_smooth(int nx, int ny, int nz, double B, double D, const 
     const size_t smem =
         (kRing + 2) * ((size_t)(kRows * L.groups + 2) * L.zl + 2) * sizeof(double);
     if ((e = cudaFuncSetAttribute(pde_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem)))
+                                  kPassShared)))
         return e;
     const dim3 grid((unsigned)tiles, (unsigned)nr);
     int s = nstep & 1;

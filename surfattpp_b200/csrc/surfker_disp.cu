@@ -433,10 +433,14 @@ template <int G>
 cudaError_t launch_groups(int nx, int ny, int nz, const double* vs3d, int nper, int runs,
                           const double* periods, int iflsph, int iwave, int igr,
                           const LayerConst* Lp, double* svel, int* status, cudaStream_t st) {
-    const int per = kGroupThreads / G, n = nx * ny;
+    constexpr int per = kGroupThreads / G;
+    const int n = nx * ny;
     const size_t bytes = per * group_bytes(nz + 1, G);
+    // (the limit belongs to the device and threads launch at the same time: the
+    // largest that any call needs, not this one's)
+    constexpr int most = (int)(per * group_bytes(sk::MMAX, G));
     cudaError_t e = cudaFuncSetAttribute(surfdisp_groups_kernel<G>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e != cudaSuccess) return e;
     surfdisp_groups_kernel<G><<<dim3((n + per - 1) / per, runs), kGroupThreads, bytes, st>>>(
         nx, ny, nz, vs3d, nper, periods, iflsph, iwave, igr, Lp, svel, status);

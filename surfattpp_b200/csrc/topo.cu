@@ -65,6 +65,7 @@ __device__ __forceinline__ double dist2_deg(double a) {
 // cell a thread, 4.5 ms so.
 constexpr int kGaussThreads = 256;
 constexpr int kGaussCells = 256;   // cells of a row at a time
+constexpr int kGaussShared = 200 * 1024;   // bytes of a block at most
 __host__ __device__ constexpr int gauss_pitch(int hx) { return (hx + 3) / 4 * 4 + 4; }
 __host__ __device__ constexpr int gauss_quarter(int nx) { return (nx + 3) / 4; }
 
@@ -344,11 +345,13 @@ cudaError_t launch_gauss_rows(int nx, int ny, int nper, const double* data, cons
     const size_t rest = 2 * (size_t)most * sizeof(double2) + 4 * kGaussCells * sizeof(double);
     int rows = 12;
     while (rows > 4 && rest + rows * row > 110 * 1024) rows -= 4;
-    while (rows > 1 && rest + rows * row > 200 * 1024) rows--;
+    while (rows > 1 && rest + rows * row > kGaussShared) rows--;
     const size_t bytes = rest + rows * row;
-    if (bytes > 200 * 1024) return cudaErrorInvalidConfiguration;   // (gauss_rows_fits)
+    if (bytes > kGaussShared) return cudaErrorInvalidConfiguration;   // (gauss_rows_fits)
+    // (the limit belongs to the device and threads launch at the same time: the
+    // largest that any call needs, not this one's)
     const cudaError_t e = cudaFuncSetAttribute(
-        gauss_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        gauss_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGaussShared);
     if (e != cudaSuccess) return e;
     gauss_rows_kernel<<<dim3(ny, nper), kGaussThreads, bytes, st>>>(nx, ny, data, lats, off, h,
                                                                     sigmas, rows, most, out);
