@@ -2267,8 +2267,9 @@ extern "C" int sa_topo_media(sa_ctx* ctx, int nx, int ny, const double* lon, con
         SA_CUDA(cudaStreamSynchronize(st));
     }
     // (the shared weights are zero beyond a window, which a topography that is
-    // not finite does not bear: such a grid is done again point by point)
-    if (!even || h_odd) {
+    // not finite does not bear: such a grid is done again point by point,
+    // unless it is too tall for that form)
+    if (!even || (h_odd && gauss_geo_fits(ny))) {
         if (const int rc = media(false)) return rc;
         SA_CUDA(cudaStreamSynchronize(st));
     }

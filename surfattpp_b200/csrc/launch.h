@@ -151,6 +151,7 @@ cudaError_t launch_model_update_vs(size_t n, const double* vs, const double* dir
                                    double* vs_out, double* vp_out, double* rho_out,
                                    cudaStream_t st);
 // topo.cu
+bool gauss_geo_fits(int ny);
 cudaError_t launch_gauss_geo(int nx, int ny, const double* data, const double* lons,
                              const double* lats, double sigma, double* out, cudaStream_t st);
 // nper (at most 65535) periods' smoothing on an evenly spaced longitude grid (step h, off =

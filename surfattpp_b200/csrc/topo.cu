@@ -326,8 +326,18 @@ __global__ void grid_kernel(int nxr, int nyr, const double* __restrict__ xr,
 }
 }  // namespace
 
+constexpr int kGeoShared = 227 * 1024;   // bytes of a block at most
+constexpr int kGeoRows = 48 * 1024 / 16;
+bool gauss_geo_fits(int ny) { return ny <= kGeoShared / 16; }
+
 cudaError_t launch_gauss_geo(int nx, int ny, const double* data, const double* lons,
                              const double* lats, double sigma, double* out, cudaStream_t st) {
+    // (set for tall grids only: up to 48 KB need no limit)
+    if (ny > kGeoRows) {
+        const cudaError_t e = cudaFuncSetAttribute(
+            gauss_geo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGeoShared);
+        if (e != cudaSuccess) return e;
+    }
     dim3 grid((nx + 127) / 128, ny);
     gauss_geo_kernel<<<grid, 128, 2 * ny * sizeof(double), st>>>(nx, ny, data, lons, lats, sigma,
                                                                  out);

@@ -1,6 +1,6 @@
 """sa_topo_media at the ends of what it accepts: windows wider than any grid,
 coordinates and topography that are not finite, more periods than a launch's
-grid holds.  Bars: media within 1e-12 and dip angles within 1e-9 degrees of
+grid holds, tall grids.  Bars: media within 1e-12 and dip angles within 1e-9 degrees of
 the oracle, the bars of the ordinary cases; non-finite values in the same
 cells as the oracle's."""
 import numpy as np
@@ -71,3 +71,14 @@ def test_more_periods_than_a_grid_holds(gpu, orc):
     _match([a[-2:] for a in got], orc.topo_media(x, y, z, sig[-2:]))
     for a in got:
         assert np.array_equal(a[0], a[65535])
+
+
+@pytest.mark.parametrize("nx,ny", [(5, 3072), (5, 3073), (131, 4001), (3, 14528)])
+def test_tall_grids(gpu, orc, nx, ny):
+    """More latitudes than the per-point form has shared memory for without
+    asking for more."""
+    x, y, z = _grid(nx, ny, 5)
+    y = 24.0 + 0.0004 * np.arange(ny)
+    z[ny // 2, nx // 2] = np.nan
+    sig = np.array([0.011])
+    _match(_media(x, y, z, sig), orc.topo_media(x, y, z, sig))
