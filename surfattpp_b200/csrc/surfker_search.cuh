@@ -117,6 +117,7 @@ struct Layers {
 template <bool TAB>
 __device__ __forceinline__ double dltar4_near(const Layers& M, double wvno, double omega) {
     const int n = M.mmax - 1;
+    if (omega < 1.0e-4) omega = 1.0e-4;   // (as dltar4 has it)
     const double w2 = wvno * wvno;
     const double io = 1.0 / omega;
     double e0, e1, e2, e3, e4;
