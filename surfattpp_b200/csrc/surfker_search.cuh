@@ -7,10 +7,12 @@
 // refinement's and the bracket ends' values are used; the march asks for
 // signs alone.  So the march evaluates dltar approximately (dltar_near: FP64
 // with short table functions, fused multiply-adds and no normalising
-// divisions, about a third of the work): its value is within 1e-9 of the
-// normalised vector's largest component of dltar's, and a sign is taken from
-// it only where it stands above 1e-6 of that; anything smaller, or not a
-// number, is evaluated exactly.  Trial velocities, brackets and Neville
+// divisions, about a third of the work): its value is within 1e-7 of the
+// normalised vector's largest component of dltar's (2e-8 the most seen at periods
+// from 1 s, next to a layer's velocity, where dltar itself cancels; 3e-11
+// elsewhere), and a sign is taken from it only where it
+// stands above 1e-6 of that; anything smaller, or not a number, is evaluated
+// exactly.  Trial velocities, brackets and Neville
 // tables are those of the Fortran, so the phase velocities are too, bit for
 // bit.
 #pragma once
@@ -77,7 +79,11 @@ __device__ __forceinline__ double pow2_rcp(double x) {
 
 // One vertical wavenumber's functions over a layer: cos and sin / r, r sin
 // (trigonometric below the layer's wavenumber, scaled hyperbolic above) and
-// the hyperbolic scale e = exp(-r d), or 1.
+// the hyperbolic scale e = exp(-r d), or 1; NaN where they are not accurate
+// enough to be trusted.  xk from rcp_near is off by 2^-46, which moves cos and
+// sin by up to (xk d)^2 2^-46 (below 1e-9 for xk d < 256); rsqrt_near moves
+// the phase p by up to p 2^-43 (1e-10 at 1e3).
+template <bool TAB>
 __device__ __forceinline__ void wave_near(double wvno, double xk, double d, double& co,
                                           double& sr, double& rs, double& e) {
     const double s = (wvno + xk) * (wvno - xk);
@@ -85,13 +91,13 @@ __device__ __forceinline__ void wave_near(double wvno, double xk, double d, doub
     const double ir = rsqrt_near(r2);
     const double r = r2 * ir;
     const double p = r * d;
+    const bool in = TAB ? s >= 0.0 || p < 1e3 : xk * d < 256.0;
     if (s < 0.0) {
         double sn;
-        const bool in = p < 1e5;
         sincos_near(in ? p : 0.0, &sn, &co);
         sr = sn * ir;
         rs = -(r * sn);
-        e = in ? 1.0 : __longlong_as_double(0x7ff8000000000000ll);
+        e = 1.0;
     } else {
         e = exp_near(-fmin(p, 700.0));
         const double f = e * e;
@@ -100,6 +106,7 @@ __device__ __forceinline__ void wave_near(double wvno, double xk, double d, doub
         sr = sn * ir;
         rs = r * sn;
     }
+    if (!in) e = __longlong_as_double(0x7ff8000000000000ll);
 }
 
 // The layers of one column as the evaluations read them: flattened REAL*4
@@ -122,8 +129,10 @@ __device__ __forceinline__ double dltar4_near(const Layers& M, double wvno, doub
     const double io = 1.0 / omega;
     double e0, e1, e2, e3, e4;
     {
-        const double xka = TAB ? M.xka[n] : omega * rcp_near(M.a[n]);
-        const double xkb = TAB ? M.xkb[n] : omega * rcp_near(M.b[n]);
+        // (quotients: ra and rb are roots of what is left of wvno next to a
+        // velocity of the half-space's, 3e-7 of it with rcp_near)
+        const double xka = TAB ? M.xka[n] : omega / (double)M.a[n];
+        const double xkb = TAB ? M.xkb[n] : omega / (double)M.b[n];
         const double ra = sqrt((wvno + xka) * fabs(wvno - xka));
         const double rb = sqrt((wvno + xkb) * fabs(wvno - xkb));
         const double t = (double)M.b[n] * io;
@@ -149,8 +158,8 @@ __device__ __forceinline__ double dltar4_near(const Layers& M, double wvno, doub
             gk = 2.0 * t * t;
         }
         double cp, w, x, ea, cq, y, z, eb;
-        wave_near(wvno, xka, d, cp, w, x, ea);
-        wave_near(wvno, xkb, d, cq, y, z, eb);
+        wave_near<TAB>(wvno, xka, d, cp, w, x, ea);
+        wave_near<TAB>(wvno, xkb, d, cq, y, z, eb);
         const double gam = gk * w2, g1 = gam - 1.0, tg = gam + g1;
         const double gmk = gam * gk, gm1 = gam * g1, g1s = g1 * g1;
         const double cpcq = cp * cq, cpy = cp * y, cpz = cp * z, cqw = cq * w, cqx = cq * x;
@@ -202,7 +211,7 @@ __device__ __forceinline__ double dltar1_near(const Layers& M, double wvno, doub
     const int n = M.mmax - 1;
     double e1, e2;
     {
-        const double ib = rcp_near(M.b[n]), xkb = TAB ? M.xkb[n] : omega * ib;
+        const double b = (double)M.b[n], ib = rcp_near(b), xkb = TAB ? M.xkb[n] : omega / b;
         e1 = (double)M.rho[n] * sqrt((wvno + xkb) * fabs(wvno - xkb));
         e2 = ib * ib;
     }
@@ -211,12 +220,13 @@ __device__ __forceinline__ double dltar1_near(const Layers& M, double wvno, doub
         const double b = (double)M.b[m], mu = (double)M.rho[m] * b * b;
         const double xkb = TAB ? M.xkb[m] : omega * rcp_near(M.b[m]);
         double co, y, z, e;
-        wave_near(wvno, xkb, (double)M.d[m], co, y, z, e);
+        wave_near<TAB>(wvno, xkb, (double)M.d[m], co, y, z, e);
         const double im = TAB ? M.rr[m] : rcp_near(mu);
         const double a = fma(e1, co, e2 * mu * z), c = fma(e1 * y, im, e2 * co);
         const double t1 = fmax(fabs(a), fabs(c));
-        if (m == 0) return M.llw == 1 ? a / t1 : t1 * __longlong_as_double(0x7ff8000000000000ll);
-        const double s = pow2_rcp(t1) * (e == e ? 1.0 : e);
+        if (!(e == e) || (m == 0 && M.llw != 1)) return __longlong_as_double(0x7ff8000000000000ll);
+        if (m == 0) return a / t1;
+        const double s = pow2_rcp(t1);
         e1 = a * s;
         e2 = c * s;
     }

@@ -2,7 +2,8 @@
 where they stand above 1e-6 of the normalised vector (kSignSure).  Host build:
 where they are trusted they lie within a tenth of that of the exact ones, in
 the form with a thread per column and in that with tables, for any trial
-velocity and for periods beyond dltar4's smallest frequency."""
+velocity, those next to a layer's or the half-space's among them, for layers of
+many wavelengths, and for periods beyond dltar4's smallest frequency."""
 import ctypes as C
 import os
 import subprocess
@@ -43,3 +44,21 @@ def _worst(lib, love, tables, where, periods, thickness, n=20_000):
 def test_any_velocity(lib, love, tables, periods):
     worst, untrusted = _worst(lib, love, tables, 0, periods, (0.3, 5.0))
     assert worst <= BOUND and untrusted < 0.01
+
+
+@pytest.mark.parametrize("love", [0, 1])
+@pytest.mark.parametrize("tables", [0, 1])
+@pytest.mark.parametrize("where", [1, 2, 3])
+def test_next_to_a_velocity(lib, love, tables, where):
+    worst, untrusted = _worst(lib, love, tables, where, (1.0, 60.0), (0.3, 5.0))
+    assert worst <= BOUND and untrusted < 0.02
+
+
+@pytest.mark.parametrize("love", [0, 1])
+@pytest.mark.parametrize("tables", [0, 1])
+@pytest.mark.parametrize("where", [0, 2])
+@pytest.mark.parametrize("periods", [(0.05, 1.0), (0.002, 0.05), (1e-4, 0.002)])
+def test_many_wavelengths(lib, love, tables, where, periods):
+    """Not trusted, or accurate."""
+    worst, _ = _worst(lib, love, tables, where, periods, (10.0, 60.0))
+    assert worst <= BOUND
