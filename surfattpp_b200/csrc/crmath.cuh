@@ -204,6 +204,9 @@ CR_HD CR_FULL_ATTR double exp_full(double x) {
 // The rounding test: s + lo (an error below eps |s|) rounds to *y whatever
 // the error is.
 CR_HD inline bool rounds_to(double s, double lo, double eps, double* y) {
+#ifdef CR_PROBE   // (the tests measure the error of s + lo)
+    CR_PROBE(s, lo, eps);
+#endif
     const double up = s + fma(s, eps, lo);
     const double dn = s + fma(s, -eps, lo);
     *y = up;
@@ -441,8 +444,9 @@ CR_HD CR_FULL_ATTR void sincos_full(double x, double* sn, double* cs) {
 // The short evaluation of both, |x| < 3216 (|kd| < 2^11) and a remainder of
 // at least 2^-20: x - kd pi/2 = h + l with kd P1, kd P2 exact products and
 // the rest of pi/2 in one double; h = j/256 + t, |t| <= 2^-9; sin t - t and
-// cos t - 1 in FP64 (below 2^-29 and 2^-18: their rounding stays below 2^-69
-// of the result), the products C t, S t error-free.
+// cos t - 1 in FP64, the products C t, S t error-free.  l reaches 2^-57 (kd
+// P3), so it enters sin(t + l) as l cos t, cos(t + l) as -l t; what is left
+// out and rounded away stays below 2^-70 of the result.
 CR_HD inline bool sincos_short(double x, double* sn, double* cs) {
     const double kd = rint(x * CR_2OPI);
     const double a = fma(-kd, CR_PIO2_1, x);
@@ -455,7 +459,7 @@ CR_HD inline bool sincos_short(double x, double* sn, double* cs) {
     const double t = fma(aj, -1.0 / 256.0, ah);   // exact
     const double z = t * t;
     const double ps = fma(z, fma(z, -CR_IFACT7, CR_IFACT5), -CR_IFACT3);
-    const double ds = fma(t * z, ps, l);                                    // sin - t
+    const double ds = fma(t * z, ps, fma(-0.5 * z, l, l));                  // sin - t
     const double pc = fma(z, fma(z, -CR_IFACT6, CR_IFACT4), -0.5);
     const double dc = fma(z, pc, -(t * l));                                 // cos - 1
     const dd S = {CR_TAB(kSinT)[2 * j], CR_TAB(kSinT)[2 * j + 1]};
