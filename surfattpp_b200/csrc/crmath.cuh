@@ -20,10 +20,10 @@
 // exp, log and sincos first run a shorter evaluation with a rounding test
 // (Ziv, ACM TOMS 17(3) 1991): the result as s + lo, taken when s + lo -+
 // eps |s| round to the same double, eps (2^-70, 2^-65, 2^-68) at least
-// twice the evaluation's error bound.  One argument in 2^16 (log 2^11, sincos
-// 2^13) fails the test and takes the full evaluation, so both give the same
-// bits; the short one takes 40 FP64 operations against 75 for exp, 56
-// against 150 for sincos and 35 against 150 for log.
+// 3.8 times the evaluation's largest measured error.  One argument in 2^16
+// (log 2^11, sincos 2^13) fails the test and takes the full evaluation, so both
+// give the same bits; the short one takes 40 FP64 operations against 75 for
+// exp, 58 against 150 for sincos and 36 against 150 for log.
 //
 // Host and device give bit-identical results: every product that is added
 // is written as an explicit fma, nothing else is contracted or reassociated
@@ -298,9 +298,9 @@ CR_HD CR_FULL_ATTR double log_full(double x) {
 }
 
 // The short evaluation of log, normal positive x: n ln2 + T_j + r - r^2/2
-// error-free, log1p(r) - r + r^2/2 = r^3 (1/3 - r/4 + ... + r^6/9) in FP64,
-// |r| <= 2^-7 (the next term is below 2^-73).  Its rounding is below 2^-75,
-// 2^-66 of the smallest result with T_j != 0 (and 2^-14 2^-52 relative where
+// error-free, log1p(r) - r + r^2/2 = r^3 (1/3 - r/4 + ... - r^7/10) in FP64,
+// |r| <= 2^-7 (the next term is below 2^-80).  What is left is the rounding of
+// r^3 (...) and of the low words' sum, at most 2^-66.9 of the result (where
 // T_j = 0, n = 0, the result being about r).
 CR_HD inline bool log_short(double x, double* y) {
     const uint64_t u = double_to_bits(x);
@@ -314,7 +314,8 @@ CR_HD inline bool log_short(double x, double* y) {
     const dd a = fast_two_sum(nl.hi, T.hi);
     const dd b = two_sum(a.hi, r);
     const dd z = two_prod(r, r);
-    double c = fma(r, 1.0 / 9.0, -1.0 / 8.0);
+    double c = fma(r, -0.1, 1.0 / 9.0);
+    c = fma(r, c, -1.0 / 8.0);
     c = fma(r, c, CR_INVODD7);
     c = fma(r, c, -1.0 / 6.0);
     c = fma(r, c, CR_INV5_HI);

@@ -50,7 +50,7 @@ def _args(f, n=60_000):
                            np.exp(g.uniform(-13, 1, n))])
 
 
-@pytest.mark.parametrize("f", [0, 2])
+@pytest.mark.parametrize("f", [0, 1, 2])
 def test_error_is_half_of_what_is_allowed(lib, f):
     x = np.ascontiguousarray(_args(f))
     at = C.c_double()
