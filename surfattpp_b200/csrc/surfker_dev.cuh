@@ -19,6 +19,7 @@
 
 #include "crmath.cuh"
 #include "launch.h"
+#include "rounded.cuh"
 
 namespace sa {
 namespace sk {
@@ -81,17 +82,6 @@ static __device__ SK_MATH_ATTR double sk_exp(double x) { return cr::exp(x); }
 static __device__ SK_MATH_ATTR double sk_log(double x) { return cr::log(x); }
 
 __device__ __forceinline__ double dsign1(double x) { return copysign(1.0, x); }
-
-// a / b rounded to nearest from rh = RN(1/b) and rl = recip_lo(b, rh), about
-// 1/b - rh: RN(a rh + a rl) lies within an ulp of a / b, its remainder is
-// exact, and one correction by rh rounds correctly (Markstein, IBM J. Res.
-// Dev. 34(1) 1990); for |a| above 2^-900 or 0.  Four operations where
-// several quotients share a divisor, against about ten of a division.
-__device__ __forceinline__ double recip_lo(double b, double rh) { return fma(-rh, b, 1.0) * rh; }
-__device__ __forceinline__ double quot(double a, double b, double rh, double rl) {
-    const double q = fma(a, rh, a * rl);
-    return fma(fma(-q, b, a), rh, q);
-}
 
 // Brocher relations, scalar forms (include/utils.h:185-187, :223-225)
 __device__ __forceinline__ double vs2vp(double vs) {

@@ -191,7 +191,7 @@ __device__ __forceinline__ double group_dltar4(const Layers& M, double* mat, int
             t1 = fmax(t1, __shfl_xor_sync(0xffffffffu, t1, 4));
             if (t1 < 1.e-40) t1 = 1.0;
             const double rh = 1.0 / t1;
-            cr = sk::quot(cr, t1, rh, sk::recip_lo(t1, rh));
+            cr = quot(cr, t1, rh, recip_lo(t1, rh));
             const double g0 = __shfl_sync(0xffffffffu, cr, base);
             const double g1 = __shfl_sync(0xffffffffu, cr, base + 1);
             const double g2 = __shfl_sync(0xffffffffu, cr, base + 2);
@@ -267,7 +267,7 @@ __device__ __forceinline__ double group_dltar1(const Layers& M, double* mat, int
             const double* o = mat + l * kMatPitch;
             const double cosq = o[0], xmu = M.r2[ml], rh = M.rr[ml];
             const double e10 = e1 * cosq + e2 * xmu * o[2];
-            const double e20 = sk::quot(e1 * o[1], xmu, rh, sk::recip_lo(xmu, rh)) + e2 * cosq;
+            const double e20 = quot(e1 * o[1], xmu, rh, recip_lo(xmu, rh)) + e2 * cosq;
             double xnor = fabs(e10);
             const double ynor = fabs(e20);
             if (ynor > xnor) xnor = ynor;
