@@ -174,11 +174,13 @@ int sa_forward_for_events(sa_ctx* ctx, int precision, int nx, int ny, int nper,
  * the plan's evaluation (arguments as sa_plan_forward_adjoint; adj_s may be
  * NULL) twice and its second batch launch is timed.  The fastest is kept by
  * the plan and by plans of the same grid size (nx, ny, precision) created
- * later on this context.  ms_out (may be NULL) receives up to
- * SA_TUNE_MAX_CANDIDATES timings, n_out the number of candidates, choice the
- * index of the one kept.  Outputs do not depend on the configuration (FP32:
- * every variant rounds the same explicit operations; adj_s up to the order
- * of its FP64 atomic sums).  Synchronises `stream`. */
+ * later on this context whose number of events takes the same form of launch
+ * (a warp per event, or the same number of warps), the slots in proportion.
+ * ms_out (may be NULL) receives up to SA_TUNE_MAX_CANDIDATES timings, n_out
+ * the number of candidates, choice the index of the one kept.  Outputs do
+ * not depend on the configuration (FP32: every variant rounds the same
+ * explicit operations; adj_s up to the order of its FP64 atomic sums).
+ * Synchronises `stream`. */
 #define SA_TUNE_MAX_CANDIDATES 32
 int sa_plan_autotune(sa_plan* plan, const double* svel, const double* m11, const double* m12,
                      const double* m22, const double* tt_obs, const double* weight,

@@ -1161,15 +1161,17 @@ inline BatchArgs<float> make_batch_args<float>(const BatchDesc& d) {
 }
 
 // Warps per event of a launch (1: batch_kernel, a warp each): as many as give
-// an SM `load` warps together, at most one per 32 rows and `most`, evened out
-// over the strips.
-inline int wide_warps(const BatchDesc& d, int load, int most) {
+// an SM `load` warps together, at most one per 32 rows and BIG / 32, evened
+// out over the strips.
+template <class S, int BIG>
+inline int wide_warps(int ny, int ne) {
+    const int load = sizeof(S) == sizeof(double) ? 10 : ny > 160 ? 14 : ny > 64 ? 10 : 4;
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int strips = (d.g.ny + 31) / 32;
-    const long long fit = (long long)load * nsm / std::max(d.ev.ne, 1);
-    const int W = (int)std::min<long long>(std::min(fit, (long long)most), strips);
+    const int strips = (ny + 31) / 32;
+    const long long fit = (long long)load * nsm / std::max(ne, 1);
+    const int W = (int)std::min<long long>(std::min<long long>(fit, BIG / 32), strips);
     if (W <= 1) return 1;
     const int turns = (strips + W - 1) / W;
     return (strips + turns - 1) / turns;
@@ -1187,8 +1189,7 @@ inline int wide_warps(const BatchDesc& d, int load, int most) {
 // 2.68 -> 2.65, 2.73 -> 3.15 (not taken).
 template <class S, int BIG>
 inline bool launch_wide(const BatchDesc& d, const double* dxdy, cudaStream_t st) {
-    const int load = sizeof(S) == sizeof(double) ? 10 : d.g.ny > 160 ? 14 : d.g.ny > 64 ? 10 : 4;
-    const int W = wide_warps(d, load, BIG / 32);
+    const int W = wide_warps<S, BIG>(d.g.ny, d.ev.ne);
     if (W <= 1 && !dxdy) return false;
     const BatchArgs<S> B = make_batch_args<S>(d);
     const int blocks = std::max(1, std::min(d.sc.nslots, d.ev.ne));

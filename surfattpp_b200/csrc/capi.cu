@@ -116,9 +116,10 @@ struct sa_ctx {
     DArr<double> red;   // reduction scratch of the optimizer entry points
     double* red_host = nullptr;   // and their results (pinned)
     std::mutex red_mutex;         // one of them at a time
-    // launch configuration chosen by sa_plan_autotune per grid size:
-    // (nx, ny, precision) -> (variant, active slots; 0 = all)
-    std::map<std::array<int, 3>, std::array<int, 2>> tune;
+    // launch configuration chosen by sa_plan_autotune per grid size and form
+    // of the launch: (nx, ny, precision, warps per event) -> (variant, quarters
+    // of the slots in use)
+    std::map<std::array<int, 4>, std::array<int, 2>> tune;
 };
 
 namespace {
@@ -640,6 +641,18 @@ int plan_enqueue(sa_plan* P, const double* svel, const double* m11, const double
 
 }  // namespace
 
+// What a tuned configuration is kept for: a choice among many events' forms
+// is no choice for few events, which a block each serves, nor the other way.
+static std::array<int, 4> tune_key(const sa_plan* P) {
+    return {P->nx, P->ny, P->prec,
+            P->prec == SA_FP64 ? batch64_event_warps(P->ny, P->ne)
+                               : batch32_event_warps(P->ny, P->ne)};
+}
+// Quarters of the event slots in use -> slots (0 = all).
+static int tune_slots(const sa_plan* P, int quarters) {
+    return quarters == 4 ? 0 : std::max(1, P->nslots * quarters / 4);
+}
+
 extern "C" int sa_plan_create(sa_ctx* ctx, int precision, int nx, int ny, int nper,
                               const double* xx_deg, const double* yy_deg, int ne,
                               const double* evlo, const double* evla, const int* iper,
@@ -665,11 +678,11 @@ extern "C" int sa_plan_create(sa_ctx* ctx, int precision, int nx, int ny, int np
         delete P;
         return rc;
     }
-    // a configuration tuned earlier for this grid size
-    const auto it = ctx->tune.find({nx, ny, precision});
+    // a configuration tuned earlier for this grid size and form
+    const auto it = ctx->tune.find(tune_key(P));
     if (it != ctx->tune.end()) {
         P->variant = it->second[0];
-        P->active = it->second[1];
+        P->active = tune_slots(P, it->second[1]);
     }
     *out = P;
     return SA_OK;
@@ -683,10 +696,10 @@ extern "C" void sa_plan_destroy(sa_plan* plan) { delete plan; }
 // slots, and with tail teams also a quarter (one solve per block).  Each
 // candidate runs the plan's own evaluation twice, the second timed with
 // CUDA events around the batch kernel; the fastest is kept for this plan and
-// for plans of the same grid size created later on this context.  Results do
-// not depend on the choice: the FP32 sweeps spell out every rounding, so all
-// variants compute the same values (only the atomic accumulation order of
-// adj_s varies).
+// for plans of the same grid size and warps per event created later on this
+// context.  Results do not depend on the choice: the FP32 sweeps spell out
+// every rounding, so all variants compute the same values (only the atomic
+// accumulation order of adj_s varies).
 extern "C" int sa_plan_autotune(sa_plan* P, const double* svel, const double* m11,
                                 const double* m12, const double* m22, const double* tt_obs,
                                 const double* weight, int calc_adj, double* adj_s,
@@ -700,13 +713,13 @@ extern "C" int sa_plan_autotune(sa_plan* P, const double* svel, const double* m1
     SA_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     const int nvar = P->prec == SA_FP32 ? kBatchVariants : 1;
-    // (variant, slots in use): all or three quarters; with tail teams also a
-    // quarter (one solve per block, its three other warps as the team)
+    // (variant, quarters of the slots in use): all or three; with tail teams
+    // also one (one solve per block, its three other warps as the team)
     std::vector<std::pair<int, int>> cand;
     for (int v = 0; v < nvar; v++) {
-        cand.push_back({v, 0});
-        cand.push_back({v, std::max(1, P->nslots * 3 / 4)});
-        if (v & 4) cand.push_back({v, std::max(1, P->nslots / 4)});
+        cand.push_back({v, 4});
+        cand.push_back({v, 3});
+        if (v & 4) cand.push_back({v, 1});
     }
     const int ncand = (int)cand.size();
     const bool had_timing = P->timing;
@@ -719,7 +732,7 @@ extern "C" int sa_plan_autotune(sa_plan* P, const double* svel, const double* m1
     int best_c = 0;
     for (int c = 0; c < ncand; c++) {
         P->variant = cand[c].first;
-        P->active = cand[c].second;
+        P->active = tune_slots(P, cand[c].second);
         float ms = 0.f;
         for (int rep = 0; rep < 2; rep++) {
             const int rc = plan_enqueue(P, svel, m11, m12, m22, tt_obs, weight, calc_adj,
@@ -739,9 +752,9 @@ extern "C" int sa_plan_autotune(sa_plan* P, const double* svel, const double* m1
     }
     P->timing = had_timing;
     P->variant = cand[best_c].first;
-    P->active = cand[best_c].second;
+    P->active = tune_slots(P, cand[best_c].second);
     P->have_graph = false;
-    ctx->tune[{P->nx, P->ny, P->prec}] = {P->variant, P->active};
+    ctx->tune[tune_key(P)] = {P->variant, cand[best_c].second};
     if (n_out) *n_out = ncand;
     if (choice) *choice = best_c;
     return SA_OK;

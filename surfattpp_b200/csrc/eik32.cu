@@ -33,6 +33,9 @@ size_t batch32_slot_bytes(int nx, int ny, int maxr) {
     return slot_layout<float>(nx, ny, maxr).total;
 }
 
+constexpr int kWide32 = 512;   // threads of an event at most
+int batch32_event_warps(int ny, int ne) { return wide_warps<float, kWide32>(ny, ne); }
+
 int batch32_max_slots(int device) {
     int nsm = 0, per_sm = 0;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
@@ -50,7 +53,7 @@ void launch_variant(const BatchDesc& d, const BatchArgs<float>& B, int blocks, c
 }  // namespace
 
 cudaError_t launch_batch32(const BatchDesc& d, cudaStream_t st) {
-    if (d.variant == 0 && launch_wide<float, 512>(d, nullptr, st)) return cudaGetLastError();
+    if (d.variant == 0 && launch_wide<float, kWide32>(d, nullptr, st)) return cudaGetLastError();
     const BatchArgs<float> B = make_batch_args<float>(d);
     // with tail teams every resident warp runs (the slots in use are spread
     // over the blocks, the other warps start as helpers)

@@ -96,6 +96,9 @@ size_t batch64_slot_bytes(int nx, int ny, int maxr) {
     return slot_layout<double>(nx, ny, maxr).total;
 }
 
+constexpr int kWide64 = 384;   // threads of an event at most
+int batch64_event_warps(int ny, int ne) { return wide_warps<double, kWide64>(ny, ne); }
+
 int batch64_max_slots(int device) {
     int nsm = 0, per_sm = 0;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
@@ -138,7 +141,7 @@ template cudaError_t launch_geometry<float>(int, int, int, const double*, const 
                                             cudaStream_t);
 
 cudaError_t launch_batch64(const BatchDesc& d, cudaStream_t st) {
-    if (launch_wide<double, 384>(d, nullptr, st)) return cudaGetLastError();
+    if (launch_wide<double, kWide64>(d, nullptr, st)) return cudaGetLastError();
     const BatchArgs<double> B = make_batch_args<double>(d);
     const int blocks = (d.sc.nslots + 3) / 4;
     if (d.iso) batch_kernel<double, true, 0><<<blocks, 128, 0, st>>>(B);
@@ -152,7 +155,7 @@ cudaError_t launch_batch64(const BatchDesc& d, cudaStream_t st) {
 // (sa_eik_fwd_field_noalloc).
 cudaError_t launch_batch64_dev_spacing(const BatchDesc& d, const double* dxdy,
                                        cudaStream_t st) {
-    launch_wide<double, 384>(d, dxdy, st);
+    launch_wide<double, kWide64>(d, dxdy, st);
     return cudaGetLastError();
 }
 

@@ -52,8 +52,10 @@ constexpr int kBatchVariants = 8;
 
 size_t batch64_slot_bytes(int nx, int ny, int maxr);
 int batch64_max_slots(int device);
+int batch64_event_warps(int ny, int ne);   // warps that a launch gives an event
 size_t batch32_slot_bytes(int nx, int ny, int maxr);
 int batch32_max_slots(int device);
+int batch32_event_warps(int ny, int ne);
 
 cudaError_t launch_media64(int nx, int ny, int nper, const double* svel, const double* m11,
                            const double* m12, const double* m22, const double* cosy,

@@ -88,7 +88,7 @@ class ForwardAdjointPlan:
                  adj_s=None, stream=None):
         """Pick the fastest batch-kernel launch configuration on this plan's own
         workload (sa_plan_autotune); kept for this plan and later plans of the
-        same grid size on its context.  Returns dict(ms=[per candidate],
+        same grid size and form of launch on its context.  Returns dict(ms=[per candidate],
         choice=index, variant, active_slots, nslots)."""
         ms = (C.c_float * 32)()
         n, ch = C.c_int(0), C.c_int(0)
