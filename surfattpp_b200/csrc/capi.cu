@@ -5,6 +5,7 @@
 // the device geometry matches a CPU evaluation bit for bit), uploads, and
 // launching / graph-replaying the device pipeline.  No numerical path of the
 // engine runs on the host.
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -2004,7 +2005,8 @@ extern "C" int sa_lbfgs_store(sa_lbfgs* L, int iter, const double* model, const 
     // the copy and the pair with the iterate before in one pass; an iterate
     // stored anew also changes the pair with the one after
     const int before = iter > 0 && L->stored_iter[(iter - 1) % R] == iter - 1 ? (iter - 1) % R : -1;
-    const int after = L->stored_iter[(iter + 1) % R] == iter + 1 ? (iter + 1) % R : -1;
+    const int next = iter < INT_MAX ? (iter + 1) % R : -1;
+    const int after = next >= 0 && L->stored_iter[next] == iter + 1 ? next : -1;
     auto pair_slot = [&](int k) { return k % R; };
     double *s0 = nullptr, *y0 = nullptr;
     if (before >= 0) {
@@ -2037,8 +2039,8 @@ extern "C" int sa_lbfgs_direction(sa_lbfgs* L, int iter, double* dir) {
     if (iter < 0 || !dir) return fail(ctx, SA_ERR_ARG, "sa_lbfgs_direction: arguments");
     const int nh = std::min(iter, LBFGS_STORE);   // src/optimize.cpp:153-154
     const int h0 = iter - nh;
-    for (int k = h0; k <= iter; k++)
-        if (L->stored_iter[k % (LBFGS_STORE + 1)] != k)
+    for (int h = 0; h <= nh; h++)
+        if (const int k = h0 + h; L->stored_iter[k % (LBFGS_STORE + 1)] != k)
             return fail(ctx, SA_ERR_ARG, "sa_lbfgs_direction: iterate " + std::to_string(k) +
                                              " was not stored");
     SA_CUDA(cudaSetDevice(ctx->device));
