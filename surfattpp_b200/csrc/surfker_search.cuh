@@ -8,13 +8,12 @@
 // signs alone.  So the march evaluates dltar approximately (dltar_near: FP64
 // with short table functions, fused multiply-adds and no normalising
 // divisions, about a third of the work): its value is within 1e-7 of the
-// normalised vector's largest component of dltar's (2e-8 the most seen at periods
-// from 1 s, next to a layer's velocity, where dltar itself cancels; 3e-11
-// elsewhere), and a sign is taken from it only where it
-// stands above 1e-6 of that; anything smaller, or not a number, is evaluated
-// exactly.  Trial velocities, brackets and Neville
-// tables are those of the Fortran, so the phase velocities are too, bit for
-// bit.
+// normalised vector's largest component of dltar's (2e-8 the most seen at
+// periods from 1 s, next to a layer's velocity, where dltar itself cancels;
+// 3e-11 elsewhere), and a sign is taken from it only where it stands above
+// 1e-6 of that; anything smaller, or not a number, is evaluated exactly.
+// Trial velocities, brackets and Neville tables are those of the Fortran, so
+// the phase velocities are too, bit for bit.
 #pragma once
 #include "surfker_dev.cuh"
 
